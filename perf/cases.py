@@ -304,6 +304,12 @@ class _Mdbas:
                         nb.as_ip(self.frozen), self.list, self.pair, self.order, self.list14,
                         self.excl, self.excl_pair)
 
+    def view(self, ptr, n):
+        """n ints of MDBas's memory as an array that keeps this owner alive."""
+        buf = (C.c_int * n).from_address(C.addressof(ptr.contents))
+        buf.owner = self
+        return np.frombuffer(buf, dtype=np.int32)
+
     def __del__(self):
         libc = C.CDLL(None)
         libc.free.argtypes = [C.c_void_p]
@@ -338,9 +344,8 @@ def run(state):
         m.energy()
         e = m.ener
         return {"force": m.force, "energy": [e.elec, e.vdw, e.virelec, e.virvdw],
-                "pair": np.ctypeslib.as_array(m.pair, (m.n,)),
-                "order": np.ctypeslib.as_array(m.order, (m.n,)),
-                "list": np.ctypeslib.as_array(m.list, (m.room,))}
+                "pair": m.view(m.pair, m.n), "order": m.view(m.order, m.n),
+                "list": m.view(m.list, m.room)}
     if f == "spme":
         e, fx, fy, fz, v = nb.spme(state["system"], ALPHA, state["grid"], state["order"])
         return {"energy": e, "force": [fx, fy, fz], "virial": v}
