@@ -11,15 +11,29 @@
 //    MDBas's dist() minimum image; neighOrder is the identity.
 //
 // Layout: after binning, positions/fractional coordinates are gathered into
-// cell order so that a warp scanning a cell reads consecutive addresses.  One
-// warp owns one atom i: lanes test 32 consecutive candidates, a ballot gives
-// the survivors and their order, so the fill pass writes j in exactly the
-// order MDBas's serial loop does.  Each builder runs a count pass, a scan
-// of the counts in neighOrder order (entry offsets) and a fill pass.
+// cell order so that a warp scanning a cell reads consecutive addresses.  Each
+// candidate pair is tested once: one warp takes eight atoms i and 32
+// consecutive candidates at a time, the test's ballot is the word of a bit
+// mask (atom, candidate), a second kernel clears the excluded pairs and
+// counts the bits, and after the scan of the counts in neighOrder order a
+// third writes the entries in bit order, which is the order MDBas's serial
+// loop visits them in.
 //
-// All distance arithmetic uses __dadd_rn/__dmul_rn (no FMA contraction) in
+// The test itself runs in FP32 on box coordinates; a pair whose FP32 r^2 lies
+// within the rounding bound of (rc+delr)^2 is settled by MDBas's FP64
+// expression, so the list is MDBas's, entry by entry.  A build of the
+// 96,000-atom box takes 0.62 ms (tests 0.31, counts 0.05, entries 0.17); FP64
+// tests, once to count and once to fill, took 2.50.  All pairs of 3,000 atoms:
+// 0.134 -> 0.072 ms.
+//
+// The FP64 arithmetic uses __dadd_rn/__dmul_rn (no FMA contraction) in
 // MDBas's association order, so every r^2 <= (rc+delr)^2 decision is the
 // one MDBas's x86 build makes.
+#include <math.h>
+
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 #include "link_stencil.h"
 #include "list_ref.cuh"
@@ -28,15 +42,15 @@ namespace mdbas {
 
 namespace {
 
+constexpr int kMaxRatio = 5;
+constexpr int kInvSide = 2 * kMaxRatio + 1;
 __constant__ int c_stencil[LINK_STENCIL_MAX * 3];
+// stencil entry of a cell offset (-5..5 per axis), -1 where there is none
+__constant__ short c_stencilOf[kInvSide * kInvSide * kInvSide];
 
-__device__ __forceinline__ bool excluded_pair(int i, int j, const int *__restrict__ exclStart,
-                                              const int *__restrict__ exclFlat) {
-  const int e = exclStart[i + 1];
-  for (int k = exclStart[i]; k < e; ++k)
-    if (__ldg(exclFlat + k) == j) return true;
-  return false;
-}
+constexpr int kGroup = 8;       // atoms i per warp of the candidate tests
+constexpr int kListWarps = 4;   // warps per block of the list kernels
+constexpr int kPiece = 32;      // candidate chunks per warp of the tests
 
 // image_update (src/utils.c:162-218), in place.
 __global__ void k_image_update(int n, DevBox b, double *x, double *y, double *z) {
@@ -123,117 +137,437 @@ __global__ void k_lc_order(int ncell, const int *__restrict__ cellStart,
   }
 }
 
-__global__ void k_lc_gather(int n, const int *__restrict__ sortedIdx,
-                            const double *__restrict__ xu, const double *__restrict__ yu,
-                            const double *__restrict__ zu, const int *__restrict__ frozen,
-                            double *__restrict__ xs, double *__restrict__ ys,
-                            double *__restrict__ zs, int *__restrict__ fs,
-                            int *__restrict__ posOf) {
+// Cell order: fractional coordinates for the exact test, FP32 box coordinates
+// (x, y, z, frozen) for the first one.  An atom more than two box lengths
+// from the origin gets NaN there: its pairs go to the exact test.
+__global__ void k_lc_gather(int ncell, DevBox b, const int *__restrict__ cellStart,
+                            const int *__restrict__ sortedIdx, const double *__restrict__ xu,
+                            const double *__restrict__ yu, const double *__restrict__ zu,
+                            const int *__restrict__ frozen, double *__restrict__ xs,
+                            double *__restrict__ ys, double *__restrict__ zs,
+                            float4 *__restrict__ cs, int *__restrict__ posOf) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
+  if (p >= cellStart[ncell]) return;
   const int i = sortedIdx[p];
-  xs[p] = xu[i];
-  ys[p] = yu[i];
-  zs[p] = zu[i];
-  fs[p] = frozen ? frozen[i] : 0;
+  const double u = xu[i], v = yu[i], w = zu[i];
+  xs[p] = u;
+  ys[p] = v;
+  zs[p] = w;
+  float4 c;
+  c.x = (float)(u * b.a1 + v * b.b1 + w * b.c1);
+  c.y = (float)(u * b.a2 + v * b.b2 + w * b.c2);
+  c.z = (float)(u * b.a3 + v * b.b3 + w * b.c3);
+  if (!(fabs(u) <= 2. && fabs(v) <= 2. && fabs(w) <= 2.)) c.x = __int_as_float(0x7fc00000);
+  c.w = frozen && frozen[i] ? 1.f : 0.f;
+  cs[p] = c;
   posOf[i] = p;
 }
 
-// One warp per atom (in neighOrder position p).  FILL=false: count entries
-// into cnt[p] and neighPair[i].  FILL=true: write them at off[p].
-template <bool FILL>
-__global__ void __launch_bounds__(256)
-k_lc_pairs(int n, DevBox b, int nlcx, int nlcy, int nlcz, int cellCheck, double cutnb2,
-           const int *__restrict__ sortedIdx, const int *__restrict__ cellOf,
-           const int *__restrict__ cellStart, const double *__restrict__ xs,
-           const double *__restrict__ ys, const double *__restrict__ zs,
-           const int *__restrict__ fs, const int *__restrict__ exclStart,
-           const int *__restrict__ exclFlat, int *__restrict__ cnt, int *__restrict__ neighPair,
-           const long long *__restrict__ off, int *__restrict__ list) {
+// Neighbour cell l of cell (ix, iy, iz) and its periodic image (in boxes).
+__device__ __forceinline__ int stencil_cell(int l, int ix, int iy, int iz, int nx, int ny, int nz,
+                                            int &sx, int &sy, int &sz) {
+  int jx = ix + c_stencil[3 * l], jy = iy + c_stencil[3 * l + 1], jz = iz + c_stencil[3 * l + 2];
+  sx = sy = sz = 0;
+  if (jx > nx - 1) { jx -= nx; sx = 1; } else if (jx < 0) { jx += nx; sx = -1; }
+  if (jy > ny - 1) { jy -= ny; sy = 1; } else if (jy < 0) { jy += ny; sy = -1; }
+  if (jz > nz - 1) { jz -= nz; sz = 1; } else if (jz < 0) { jz += nz; sz = -1; }
+  return jx + nx * (jy + ny * jz);
+}
+
+// Candidate chunks of every cell, one warp per cell: chunkOff[l], the first
+// chunk of stencil cell l (its atoms in runs of 32), chunkOff[cellCheck] the
+// total, and chunkBase[c], the first position of chunk c.  A total beyond
+// stride raises FLAG_CELL and goes to *need.
+__global__ void __launch_bounds__(32 * kListWarps)
+k_lc_chunks(int ncell, int nx, int ny, int nz, int cellCheck, int stride,
+            const int *__restrict__ cellStart, int *__restrict__ chunkOff,
+            int *__restrict__ chunkBase, int *__restrict__ flags, int *__restrict__ need) {
   const int lane = threadIdx.x & 31;
-  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (p >= n) return;
-  const int i = sortedIdx[p];
-  const int k = cellOf[i];
-  const int ix = k % nlcx, iy = (k / nlcx) % nlcy, iz = k / (nlcx * nlcy);
-  const double xi = xs[p], yi = ys[p], zi = zs[p];
-  const int fi = fs[p];
-  long long out = FILL ? off[p] : 0;
-  int count = 0;
-  for (int l = 0; l < cellCheck; ++l) {
-    int jx = ix + c_stencil[3 * l], jy = iy + c_stencil[3 * l + 1], jz = iz + c_stencil[3 * l + 2];
-    double cx = 0., cy = 0., cz = 0.;
-    if (jx > nlcx - 1) { jx -= nlcx; cx = 1.; } else if (jx < 0) { jx += nlcx; cx = -1.; }
-    if (jy > nlcy - 1) { jy -= nlcy; cy = 1.; } else if (jy < 0) { jy += nlcy; cy = -1.; }
-    if (jz > nlcz - 1) { jz -= nlcz; cz = 1.; } else if (jz < 0) { jz += nlcz; cz = -1.; }
-    const int ll = jx + nlcx * (jy + nlcy * jz);
-    const int lo = (ll == k) ? p + 1 : cellStart[ll];
-    const int hi = cellStart[ll + 1];
-    for (int base = lo; base < hi; base += 32) {
-      const int q = base + lane;
-      bool pass = false;
-      int j = -1;
-      if (q < hi) {
-        j = sortedIdx[q];
-        const double xt = dadd(dsub(xs[q], xi), cx);
-        const double yt = dadd(dsub(ys[q], yi), cy);
-        const double zt = dadd(dsub(zs[q], zi), cz);
-        const double xd = dadd(dadd(dmul(xt, b.a1), dmul(yt, b.b1)), dmul(zt, b.c1));
-        const double yd = dadd(dadd(dmul(xt, b.a2), dmul(yt, b.b2)), dmul(zt, b.c2));
-        const double zd = dadd(dadd(dmul(xt, b.a3), dmul(yt, b.b3)), dmul(zt, b.c3));
-        const double r2 = dadd(dadd(dmul(xd, xd), dmul(yd, yd)), dmul(zd, zd));
-        pass = (r2 <= cutnb2) && (fi * fs[q] == 0) && !excluded_pair(i, j, exclStart, exclFlat);
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, pass);
-      if (FILL && pass) list[out + __popc(m & ((1u << lane) - 1u))] = j;
-      out += __popc(m);
-      count += __popc(m);
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (k >= ncell) return;
+  const int ix = k % nx, iy = (k / nx) % ny, iz = k / (nx * ny);
+  int *off = chunkOff + (size_t)k * (cellCheck + 1);
+  int *base = chunkBase + (size_t)k * stride;
+  int run = 0;
+  for (int l0 = 0; l0 < cellCheck; l0 += 32) {
+    const int l = l0 + lane;
+    int lo = 0, nc = 0;
+    if (l < cellCheck) {
+      int sx, sy, sz;
+      const int ll = stencil_cell(l, ix, iy, iz, nx, ny, nz, sx, sy, sz);
+      lo = cellStart[ll];
+      nc = (cellStart[ll + 1] - lo + 31) >> 5;
     }
+    int x = nc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (l < cellCheck) {
+      const int first = run + x - nc;
+      off[l] = first;
+      for (int c = 0; c < nc && first + c < stride; ++c) base[first + c] = lo + 32 * c;
+    }
+    run += __shfl_sync(0xffffffffu, x, 31);
   }
-  if (!FILL && lane == 0) {
-    cnt[p] = count;
-    neighPair[i] = count;
+  if (lane == 0) {
+    off[cellCheck] = run;
+    if (run > stride) {
+      atomicOr(flags, FLAG_CELL);
+      atomicMax(need, run);
+    }
   }
 }
 
-// All-pairs builder: one warp per atom i < n-1, candidates j = i+1..n-1.
-template <bool FILL>
-__global__ void __launch_bounds__(256)
-k_vl_pairs(int n, DevBox b, double cutnb2, const double *__restrict__ x,
-           const double *__restrict__ y, const double *__restrict__ z,
-           const int *__restrict__ frozen, const int *__restrict__ exclStart,
-           const int *__restrict__ exclFlat, int *__restrict__ cnt, int *__restrict__ neighPair,
-           const long long *__restrict__ off, int *__restrict__ list) {
+// Where the candidates of atom p lie: chunks [first, last) of its mask row.
+// Link cells: atoms are tested in runs, the part of a group of kGroup
+// consecutive positions that lies in one cell; chunks of the own cell before
+// the run hold no candidate.  All pairs: chunk c is atoms 32c .. 32c + 31.
+struct ChunkMap {
+  int linkCells, n, stride, cellCheck, ncell, nlc[3];
+  const int *cellStart, *cellOf, *order, *posOf, *chunkOff, *chunkBase;
+
+  __device__ __forceinline__ int atoms() const { return linkCells ? cellStart[ncell] : n; }
+  __device__ __forceinline__ int atom(int p) const { return linkCells ? order[p] : p; }
+  __device__ __forceinline__ void range(int p, int cell, int &first, int &last) const {
+    const int g0 = p & ~(kGroup - 1);
+    if (linkCells) {
+      const int s = cellStart[cell];
+      first = (max(g0, s) + 1 - s) >> 5;
+      last = chunkOff[(size_t)cell * (cellCheck + 1) + cellCheck];
+    } else {
+      first = (g0 + 1) >> 5;
+      last = (n + 31) >> 5;
+    }
+  }
+};
+
+// The row words of up to kGroup atoms, kept one per lane until four chunks
+// are done: lane 4 g + c holds word c of atom g, so a store writes 16 bytes
+// of every row.
+struct RowWords {
+  unsigned word = 0;
+  __device__ __forceinline__ void put(int lane, int g, int c, unsigned m) {
+    if (lane == 4 * g + (c & 3)) word = m;
+  }
+  __device__ __forceinline__ void flush(int lane, int c, int atoms, unsigned *rows, int stride) {
+    const int g = lane >> 2;
+    if (g < atoms) rows[(size_t)g * stride + (c & ~3) + (lane & 3)] = word;
+    word = 0;
+  }
+};
+
+// Bits of a chunk starting at `base` that come after position p.
+__device__ __forceinline__ unsigned bits_after(int p, int base) {
+  const int s = p - base;
+  return s < 0 ? 0xffffffffu : s >= 31 ? 0u : 0xffffffffu << (s + 1);
+}
+
+// Candidate tests, link cells: one warp per group of kGroup positions in
+// [p0, p1) (p0 a multiple of kGroup) and piece of kPiece chunks (grid y); rows
+// of masks start at p0.
+// rl2 = (rc+delr)^2; band bounds the error of the FP32 r^2 near rl2.
+// Bound by instruction issue: per candidate word 6 FP32 operations, two
+// compares and a ballot, the candidate's load shared by the group.  (Boxes
+// around the chunks, to skip those out of reach, took away a fifth of the
+// tests' instructions and gave it back in the boxes' own kernels.)
+template <bool FROZEN>
+__global__ void __launch_bounds__(32 * kListWarps)
+k_lc_masks(int p0, int p1, DevBox b, ChunkMap map, double cutnb2, float rl2, float band,
+           const double *__restrict__ xs, const double *__restrict__ ys,
+           const double *__restrict__ zs, const float4 *__restrict__ cs,
+           const int *__restrict__ flags, unsigned *__restrict__ masks) {
   const int lane = threadIdx.x & 31;
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int g0 = p0 + kGroup * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int end = min(min(g0 + kGroup, p1), map.atoms());
+  if (g0 >= end || (*flags & FLAG_CELL)) return;
+  const int nx = map.nlc[0], ny = map.nlc[1], nz = map.nlc[2];
+  for (int p = g0; p < end;) {
+    const int k = map.cellOf[map.order[p]];
+    const int ix = k % nx, iy = (k / nx) % ny, iz = k / (nx * ny);
+    const int atoms = min(map.cellStart[k + 1], end) - p;
+    float x[kGroup], y[kGroup], z[kGroup];
+    unsigned frozenRows = 0;
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g) {
+      // rows that are not there: far from everything
+      x[g] = 1e18f;
+      y[g] = z[g] = 0.f;
+      if (g < atoms) {
+        const float4 c = cs[p + g];
+        x[g] = c.x;
+        y[g] = c.y;
+        z[g] = c.z;
+        if (FROZEN && c.w != 0.f) frozenRows |= 1u << g;
+      }
+    }
+    unsigned *rows = masks + (size_t)(p - p0) * map.stride;
+    // this warp's piece of the chunks, from the first that holds a position
+    // after p
+    const int *off = map.chunkOff + (size_t)k * (map.cellCheck + 1);
+    const int cFirst = max((p + 1 - map.cellStart[k]) >> 5, (int)blockIdx.y * kPiece);
+    const int cLast = min(off[map.cellCheck], (int)(blockIdx.y + 1) * kPiece);
+    if (cFirst >= cLast) {
+      p += atoms;
+      continue;
+    }
+    RowWords words;
+    int c = cFirst;
+    // the chunks of stencil cell l; OWN: the cell itself, where only
+    // positions after atom p + g count
+    const auto scan = [&](int l, auto own) {
+      constexpr bool OWN = decltype(own)::value;
+      int sx, sy, sz;
+      const int ll = stencil_cell(l, ix, iy, iz, nx, ny, nz, sx, sy, sz);
+      const float ox = (float)(sx * b.a1 + sy * b.b1 + sz * b.c1);
+      const float oy = (float)(sx * b.a2 + sy * b.b2 + sz * b.c2);
+      const float oz = (float)(sx * b.a3 + sy * b.b3 + sz * b.c3);
+      const int hi = map.cellStart[ll + 1];
+      int base = map.cellStart[ll] + 32 * (c - off[l]);
+      for (; base < hi && c < cLast; base += 32, ++c) {
+        const int q = base + lane;
+        float4 d = make_float4(-1e18f, 0.f, 0.f, 0.f);
+        if (q < hi) d = cs[q];
+        d.x += ox;
+        d.y += oy;
+        d.z += oz;
+        bool unsure = false;
+        // atoms i that make a pair of two frozen atoms with this candidate
+        const unsigned skip = FROZEN && d.w != 0.f ? frozenRows : 0u;
+#pragma unroll
+        for (int g = 0; g < kGroup; ++g) {
+          const float dx = d.x - x[g], dy = d.y - y[g], dz = d.z - z[g];
+          const float t = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, -rl2)));
+          unsure |= !(fabsf(t) > band);
+          unsigned m = __ballot_sync(0xffffffffu, t <= 0.f && !(FROZEN && (skip >> g & 1u)));
+          if (OWN) m &= bits_after(p + g, base);
+          words.put(lane, g, c, m);
+        }
+        if (__any_sync(0xffffffffu, unsure)) {
+          double xq = 0., yq = 0., zq = 0.;
+          if (q < hi) {
+            xq = xs[q];
+            yq = ys[q];
+            zq = zs[q];
+          }
+          for (int g = 0; g < atoms; ++g) {
+            const float4 ci = cs[p + g];
+            const float dx = d.x - ci.x, dy = d.y - ci.y, dz = d.z - ci.z;
+            const float t = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, -rl2)));
+            bool pass = q < hi && t <= 0.f;
+            if (q < hi && !(fabsf(t) > band)) {
+              const double xt = dadd(dsub(xq, xs[p + g]), (double)sx);
+              const double yt = dadd(dsub(yq, ys[p + g]), (double)sy);
+              const double zt = dadd(dsub(zq, zs[p + g]), (double)sz);
+              const double xd = dadd(dadd(dmul(xt, b.a1), dmul(yt, b.b1)), dmul(zt, b.c1));
+              const double yd = dadd(dadd(dmul(xt, b.a2), dmul(yt, b.b2)), dmul(zt, b.c2));
+              const double zd = dadd(dadd(dmul(xt, b.a3), dmul(yt, b.b3)), dmul(zt, b.c3));
+              pass = dadd(dadd(dmul(xd, xd), dmul(yd, yd)), dmul(zd, zd)) <= cutnb2;
+            }
+            if (FROZEN && (skip >> g & 1u)) pass = false;
+            unsigned m = __ballot_sync(0xffffffffu, pass);
+            if (OWN) m &= bits_after(p + g, base);
+            words.put(lane, g, c, m);
+          }
+        }
+        if ((c & 3) == 3) words.flush(lane, c, atoms, rows, map.stride);
+      }
+    };
+    int l = 0;
+    while (l < map.cellCheck && off[l + 1] <= c) ++l;
+    if (l == 0 && c < cLast) {
+      scan(0, std::true_type{});
+      l = 1;
+    }
+    for (; l < map.cellCheck && c < cLast; ++l) scan(l, std::false_type{});
+    if (c & 3) words.flush(lane, c, atoms, rows, map.stride);
+    p += atoms;
+  }
+}
+
+// FP32 coordinates of the all-pairs tests: the atom wrapped into the box
+// (NaN, so the exact test, when it lies absurdly far out), and frozen.
+__global__ void k_vl_coords(int n, double lx, double ly, double lz, const double *__restrict__ x,
+                            const double *__restrict__ y, const double *__restrict__ z,
+                            const int *__restrict__ frozen, float4 *__restrict__ cs,
+                            int *__restrict__ order) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double xi = x[i], yi = y[i], zi = z[i];
-  const int fi = frozen ? frozen[i] : 0;
-  long long out = FILL ? off[i] : 0;
-  int count = 0;
-  for (int base = i + 1; base < n; base += 32) {
-    const int j = base + lane;
-    bool pass = false;
-    if (j < n) {
-      double dx = dsub(x[j], xi), dy = dsub(y[j], yi), dz = dsub(z[j], zi);
-      const double r2 = dist_d(b, dx, dy, dz);
-      const int fj = frozen ? frozen[j] : 0;
-      pass = (r2 <= cutnb2) && (fi * fj == 0) && !excluded_pair(i, j, exclStart, exclFlat);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, pass);
-    if (FILL && pass) list[out + __popc(m & ((1u << lane) - 1u))] = j;
-    out += __popc(m);
-    count += __popc(m);
+  float4 c;
+  c.x = (float)(xi - lx * rint(xi / lx));
+  c.y = (float)(yi - ly * rint(yi / ly));
+  c.z = (float)(zi - lz * rint(zi / lz));
+  if (!(fabs(xi) <= 1e6 * lx && fabs(yi) <= 1e6 * ly && fabs(zi) <= 1e6 * lz))
+    c.x = __int_as_float(0x7fc00000);
+  c.w = frozen && frozen[i] ? 1.f : 0.f;
+  cs[i] = c;
+  order[i] = i;
+}
+
+// Candidate tests, all pairs: one warp per group of kGroup atoms and piece of
+// kPiece chunks (grid y), candidates j > i in index order.  The FP32
+// distance takes per axis the smaller of |d| and L - |d| (both atoms in the
+// box); exactOnly: boxes without that form take dist() for every pair.
+template <bool FROZEN>
+__global__ void __launch_bounds__(32 * kListWarps)
+k_vl_masks(int p0, int p1, DevBox b, ChunkMap map, double cutnb2, float rl2, float band, float lx,
+           float ly, float lz, int exactOnly, const double *__restrict__ xd,
+           const double *__restrict__ yd, const double *__restrict__ zd,
+           const float4 *__restrict__ cs, unsigned *__restrict__ masks) {
+  const int lane = threadIdx.x & 31;
+  const int p = p0 + kGroup * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int n = map.n, atoms = min(p + kGroup, p1) - p;
+  if (atoms <= 0) return;
+  const int cEnd = min((int)(blockIdx.y + 1) * kPiece, (n + 31) >> 5);
+  const int cFirst = max((p + 1) >> 5, (int)blockIdx.y * kPiece);
+  if (cFirst >= cEnd) return;
+  float x[kGroup], y[kGroup], z[kGroup];
+  unsigned frozenRows = 0;
+#pragma unroll
+  for (int g = 0; g < kGroup; ++g) {
+    const float4 c = cs[min(p + g, n - 1)];
+    x[g] = c.x;
+    y[g] = c.y;
+    z[g] = c.z;
+    if (FROZEN && c.w != 0.f) frozenRows |= 1u << g;
   }
-  if (!FILL && lane == 0) {
-    cnt[i] = count;
-    neighPair[i] = count;
+  unsigned *rows = masks + (size_t)(p - p0) * map.stride;
+  RowWords words;
+  int c = cFirst;
+  for (; c < cEnd; ++c) {
+    const int base = 32 * c, q = base + lane;
+    const float4 d = cs[min(q, n - 1)];
+    bool unsure = exactOnly != 0;
+    const unsigned skip = FROZEN && d.w != 0.f ? frozenRows : 0u;
+    const unsigned there = n - base >= 32 ? 0xffffffffu : (1u << (n - base)) - 1u;
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g) {
+      float dx = fabsf(d.x - x[g]), dy = fabsf(d.y - y[g]), dz = fabsf(d.z - z[g]);
+      dx = fminf(dx, lx - dx);
+      dy = fminf(dy, ly - dy);
+      dz = fminf(dz, lz - dz);
+      const float t = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, -rl2)));
+      unsure |= !(fabsf(t) > band);
+      const unsigned m = __ballot_sync(0xffffffffu, t <= 0.f && !(FROZEN && (skip >> g & 1u)));
+      words.put(lane, g, c, m & there & bits_after(p + g, base));
+    }
+    if (__any_sync(0xffffffffu, unsure)) {
+      double xq = 0., yq = 0., zq = 0.;
+      if (q < n) {
+        xq = xd[q];
+        yq = yd[q];
+        zq = zd[q];
+      }
+      for (int g = 0; g < atoms; ++g) {
+        const float4 ci = cs[p + g];
+        float dx = fabsf(d.x - ci.x), dy = fabsf(d.y - ci.y), dz = fabsf(d.z - ci.z);
+        dx = fminf(dx, lx - dx);
+        dy = fminf(dy, ly - dy);
+        dz = fminf(dz, lz - dz);
+        const float t = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, -rl2)));
+        bool pass = t <= 0.f;
+        if (q < n && (exactOnly || !(fabsf(t) > band))) {
+          double ex = dsub(xq, xd[p + g]), ey = dsub(yq, yd[p + g]), ez = dsub(zq, zd[p + g]);
+          pass = dist_d(b, ex, ey, ez) <= cutnb2;
+        }
+        if (FROZEN && (skip >> g & 1u)) pass = false;
+        const unsigned m = __ballot_sync(0xffffffffu, pass);
+        words.put(lane, g, c, m & there & bits_after(p + g, base));
+      }
+    }
+    if ((c & 3) == 3) words.flush(lane, c, atoms, rows, map.stride);
+  }
+  if (c & 3) words.flush(lane, c, atoms, rows, map.stride);
+}
+
+// One warp per atom of [p0, p1): the pairs that the atom's exclusion row
+// names are cleared from its mask row and the bits that are left counted.
+__global__ void __launch_bounds__(32 * kListWarps)
+k_list_count(int p0, int p1, ChunkMap map, const int *__restrict__ exclStart,
+             const int *__restrict__ exclFlat, const int *__restrict__ flags, unsigned *masks,
+             int *__restrict__ cnt, int *__restrict__ neighPair) {
+  const int lane = threadIdx.x & 31;
+  const int p = p0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (p >= min(p1, map.atoms()) || (*flags & FLAG_CELL)) return;
+  const int i = map.atom(p);
+  unsigned *row = masks + (size_t)(p - p0) * map.stride;
+  const int cell = map.linkCells ? map.cellOf[i] : 0;
+  const int nx = map.nlc[0], ny = map.nlc[1], nz = map.nlc[2];
+  for (int e = exclStart[i] + lane; e < exclStart[i + 1]; e += 32) {
+    const int j = exclFlat[e];
+    if ((unsigned)j >= (unsigned)map.n) continue;
+    if (!map.linkCells) {
+      if (j > i) atomicAnd(row + (j >> 5), ~(1u << (j & 31)));
+      continue;
+    }
+    const int kj = map.cellOf[j];
+    if (kj < 0) continue;
+    // offset of j's cell in the stencil, by the shorter way round
+    int dx = kj % nx - cell % nx, dy = (kj / nx) % ny - (cell / nx) % ny,
+        dz = kj / (nx * ny) - cell / (nx * ny);
+    if (2 * dx > nx) dx -= nx; else if (2 * dx < -nx) dx += nx;
+    if (2 * dy > ny) dy -= ny; else if (2 * dy < -ny) dy += ny;
+    if (2 * dz > nz) dz -= nz; else if (2 * dz < -nz) dz += nz;
+    if (abs(dx) > kMaxRatio || abs(dy) > kMaxRatio || abs(dz) > kMaxRatio) continue;
+    const int l = c_stencilOf[((dz + kMaxRatio) * kInvSide + dy + kMaxRatio) * kInvSide + dx +
+                              kMaxRatio];
+    if (l < 0 || l >= map.cellCheck) continue;
+    const int o = map.posOf[j] - map.cellStart[kj];
+    atomicAnd(row + map.chunkOff[(size_t)cell * (map.cellCheck + 1) + l] + (o >> 5),
+              ~(1u << (o & 31)));
+  }
+  __syncwarp();
+  int first, last, total = 0;
+  map.range(p, cell, first, last);
+  for (int c = first + lane; c < last; c += 32) total += __popc(__ldcg(row + c));
+  total = __reduce_add_sync(0xffffffffu, total);
+  if (lane == 0) {
+    cnt[p] = total;
+    neighPair[i] = total;
   }
 }
 
-__global__ void k_iota(int n, int *v) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = i;
+// One warp per atom of [p0, p1): its entries at off[p], in bit order.  32
+// words at a time are spread into shared memory, one lane per word, and
+// copied out in consecutive addresses.
+__global__ void __launch_bounds__(32 * kListWarps)
+k_list_fill(int p0, int p1, ChunkMap map, const unsigned *__restrict__ masks,
+            const long long *__restrict__ off, int *__restrict__ list) {
+  __shared__ int buf[kListWarps][1024];
+  const int lane = threadIdx.x & 31;
+  const int p = p0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (p >= p1) return;
+  int *const b = buf[threadIdx.x >> 5];
+  const unsigned *row = masks + (size_t)(p - p0) * map.stride;
+  const int cell = map.linkCells ? map.cellOf[map.order[p]] : 0;
+  const int *bases = map.chunkBase + (size_t)cell * map.stride;
+  int first, last;
+  map.range(p, cell, first, last);
+  int *out = list + off[p];
+  for (int c0 = first; c0 < last; c0 += 32) {
+    const int c = c0 + lane;
+    unsigned m = c < last ? row[c] : 0u;
+    const int base = map.linkCells ? (c < last ? bases[c] : 0) : 32 * c;
+    const int own = __popc(m);
+    int x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, x, 31);
+    for (int o = x; m;) {  // from the top bit down
+      const int bit = 31 - __clz(m);
+      m ^= 1u << bit;
+      b[--o] = base + bit;
+    }
+    __syncwarp();
+    for (int e = lane; e < total; e += 32) out[e] = map.linkCells ? map.order[b[e]] : b[e];
+    __syncwarp();
+    out += total;
+  }
 }
 
 __global__ void k_gather_counts(int n, const int *__restrict__ order,
@@ -252,14 +586,25 @@ int load_stencil() {
   for (int l = 0; l < LINK_STENCIL_MAX; ++l)
     for (int d = 0; d < 3; ++d) flat[3 * l + d] = LINK_STENCIL[l][d];
   MDB_CUDA(cudaMemcpyToSymbol(c_stencil, flat, sizeof(flat)));
+  short of[kInvSide * kInvSide * kInvSide];
+  for (short &v : of) v = -1;
+  for (int l = 0; l < LINK_STENCIL_MAX; ++l)
+    of[((LINK_STENCIL[l][2] + kMaxRatio) * kInvSide + LINK_STENCIL[l][1] + kMaxRatio) * kInvSide +
+       LINK_STENCIL[l][0] + kMaxRatio] = (short)l;
+  MDB_CUDA(cudaMemcpyToSymbol(c_stencilOf, of, sizeof(of)));
   if (dev >= 0 && dev < 64) g_stencil_loaded[dev] = true;
   return MDBAS_NB_OK;
 }
 
-int read_flags(const int *dflags, cudaStream_t s, int *h) {
-  MDB_CUDA(cudaMemcpyAsync(h, dflags, sizeof(int), cudaMemcpyDeviceToHost, s));
-  MDB_CUDA(cudaStreamSynchronize(s));
-  return MDBAS_NB_OK;
+// Mask rows of at most this size are kept at a time; larger systems are
+// tested in slabs of atoms, once to count and once to fill.
+constexpr size_t kMaskBytes = (size_t)1 << 30;
+
+// Bound of the FP32 test's error in r^2 near rl^2 when the coordinates' and
+// shifts' roundings add up to `err` per axis (sum over the three axes by
+// Cauchy-Schwarz, a quarter on top), with the roundings of the sum itself.
+float test_band(double rl, double err) {
+  return (float)(2.0 * 1.7320508 * rl * err * 1.25 + rl * rl / 2097152.0);
 }
 
 }  // namespace
@@ -300,97 +645,157 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
   }
   const double cutnb = cutOff + delr;
   const double cutnb2 = cutnb * cutnb;
+  const double ulp = 1.0 / 16777216.0;  // half an FP32 ulp, relative
   w.linkCells = linkCells;
   MDB_TRY(w.neighPair.ensure(sizeof(int) * n));
   MDB_TRY(w.order.ensure(sizeof(int) * n));
   MDB_TRY(w.cnt.ensure(sizeof(int) * n));
-  MDB_TRY(w.off.ensure(sizeof(long long) * (n + 1)));
-  MDB_TRY(w.scanTmp.ensure(scan_tmp_bytes(n + 1)));
-  MDB_TRY(w.flags.ensure(sizeof(int) * 4));
-  MDB_CUDA(cudaMemsetAsync(w.flags.p, 0, sizeof(int) * 4, s));
+  // the flags (error bits, chunks needed) sit behind the entry total, so that
+  // one copy brings back both
+  MDB_TRY(w.off.ensure(sizeof(long long) * (n + 2)));
+  int *flags = reinterpret_cast<int *>(w.off.as<long long>() + n + 1);
+  MDB_TRY(w.cs.ensure(sizeof(float4) * n));
 
+  ChunkMap map{};
+  map.linkCells = linkCells;
+  map.n = n;
+  int ratio = 1;
   if (linkCells) {
     MDB_TRY(load_stencil());
-    int r = linkRatio < 1 ? 1 : (linkRatio > 5 ? 5 : linkRatio);
-    link_cell_dims(b, cutOff, delr, r, w.nlc);
-    if (w.nlc[0] < 2 * r + 1 || w.nlc[1] < 2 * r + 1 || w.nlc[2] < 2 * r + 1)
+    ratio = linkRatio < 1 ? 1 : (linkRatio > kMaxRatio ? kMaxRatio : linkRatio);
+    link_cell_dims(b, cutOff, delr, ratio, w.nlc);
+    if (w.nlc[0] < 2 * ratio + 1 || w.nlc[1] < 2 * ratio + 1 || w.nlc[2] < 2 * ratio + 1)
       return MDBAS_NB_ERR_LINKCELL;  // LNKCELL_NCELLS_ERROR, src/list.c:1900-1908
-    const int ncell = w.nlc[0] * w.nlc[1] * w.nlc[2];
-    w.ncell = ncell;
-    const int cellCheck = LINK_STENCIL_COUNT[r - 1];
+    w.ncell = w.nlc[0] * w.nlc[1] * w.nlc[2];
+    map.ncell = w.ncell;
+    for (int d = 0; d < 3; ++d) map.nlc[d] = w.nlc[d];
+    map.cellCheck = LINK_STENCIL_COUNT[ratio - 1];
+    // chunks per cell of evenly spread atoms with room for fluctuations; a
+    // denser cell reports what it needs and the build is made again
+    const double per = (double)n / w.ncell;
+    map.stride = map.cellCheck * (int)((1.25 * per + 3. * sqrt(per)) / 32. + 1.);
+    map.stride = (std::max(map.stride, w.maskStride) + 3) & ~3;
+  } else {
+    w.ncell = 0;
+    map.stride = (((n + 31) >> 5) + 3) & ~3;
+  }
+  MDB_TRY(w.scanTmp.ensure(std::max(scan_tmp_bytes(w.ncell + 1), scan_tmp_bytes(n + 1))));
+  const int ncell = w.ncell;
+  if (linkCells) {
     MDB_TRY(w.xu.ensure(sizeof(double) * n));
     MDB_TRY(w.yu.ensure(sizeof(double) * n));
     MDB_TRY(w.zu.ensure(sizeof(double) * n));
     MDB_TRY(w.xs.ensure(sizeof(double) * n));
     MDB_TRY(w.ys.ensure(sizeof(double) * n));
     MDB_TRY(w.zs.ensure(sizeof(double) * n));
-    MDB_TRY(w.fs.ensure(sizeof(int) * n));
     MDB_TRY(w.cellOf.ensure(sizeof(int) * n));
     MDB_TRY(w.posOf.ensure(sizeof(int) * n));
     MDB_TRY(w.tmpIdx.ensure(sizeof(int) * n));
-    MDB_TRY(w.cellCount.ensure(sizeof(int) * (ncell + 1)));
-    MDB_TRY(w.cellFill.ensure(sizeof(int) * (ncell + 1)));
+    // counts and fill marks side by side: cleared together
+    MDB_TRY(w.cellCount.ensure(sizeof(int) * 2 * (size_t)(ncell + 1)));
     MDB_TRY(w.cellStart.ensure(sizeof(int) * (ncell + 2)));
-    MDB_TRY(w.scanTmp.ensure(scan_tmp_bytes(ncell + 1) > scan_tmp_bytes(n + 1)
-                                 ? scan_tmp_bytes(ncell + 1)
-                                 : scan_tmp_bytes(n + 1)));
-    MDB_CUDA(cudaMemsetAsync(w.cellCount.p, 0, sizeof(int) * (ncell + 1), s));
-    MDB_CUDA(cudaMemsetAsync(w.cellFill.p, 0, sizeof(int) * (ncell + 1), s));
-    MDB_LAUNCH(k_lc_bin, grid_for(n, 256), 256, 0, s, n, b, w.nlc[0], w.nlc[1], w.nlc[2], x, y,
-               z, w.xu.as<double>(), w.yu.as<double>(), w.zu.as<double>(), w.cellOf.as<int>(),
-               w.cellCount.as<int>(), w.flags.as<int>());
-    int hflags = 0;
-    MDB_TRY(read_flags(w.flags.as<int>(), s, &hflags));
-    if (hflags & FLAG_NONFINITE) return MDBAS_NB_ERR_NONFINITE;
-    if (hflags & FLAG_OUTSIDE) return MDBAS_NB_ERR_BOX;
-    MDB_TRY(exclusive_scan32(w.cellCount.as<int>(), w.cellStart.as<int>(), ncell,
-                             w.scanTmp.p, s));
-    MDB_LAUNCH(k_lc_scatter, grid_for(n, 256), 256, 0, s, n, w.cellOf.as<int>(),
-               w.cellStart.as<int>(), w.cellFill.as<int>(), w.tmpIdx.as<int>());
-    MDB_LAUNCH(k_lc_order, ncell, 256, 0, s, ncell, w.cellStart.as<int>(), w.tmpIdx.as<int>(),
-               w.order.as<int>());
-    MDB_LAUNCH(k_lc_gather, grid_for(n, 256), 256, 0, s, n, w.order.as<int>(), w.xu.as<double>(),
-               w.yu.as<double>(), w.zu.as<double>(), frozen, w.xs.as<double>(),
-               w.ys.as<double>(), w.zs.as<double>(), w.fs.as<int>(), w.posOf.as<int>());
-    const int blocks = grid_for((long long)n * 32, 256);
-    MDB_LAUNCH(k_lc_pairs<false>, blocks, 256, 0, s, n, b, w.nlc[0], w.nlc[1], w.nlc[2],
-               cellCheck, cutnb2, w.order.as<int>(), w.cellOf.as<int>(), w.cellStart.as<int>(),
-               w.xs.as<double>(), w.ys.as<double>(), w.zs.as<double>(), w.fs.as<int>(),
-               exclStart, exclFlat, w.cnt.as<int>(), w.neighPair.as<int>(),
-               (const long long *)nullptr, (int *)nullptr);
-    MDB_TRY(exclusive_scan(w.cnt.as<int>(), w.off.as<long long>(), n, w.scanTmp.p, s));
-    long long total = 0;
-    MDB_CUDA(cudaMemcpyAsync(&total, w.off.as<long long>() + n, sizeof(long long),
-                             cudaMemcpyDeviceToHost, s));
-    MDB_CUDA(cudaStreamSynchronize(s));
-    w.entries = total;
-    if (total > 0x7fffffffLL) return MDBAS_NB_ERR_CAPACITY;  // MDBas's int list index
-    MDB_TRY(w.list.ensure(sizeof(int) * (size_t)(total > 0 ? total : 1)));
-    MDB_LAUNCH(k_lc_pairs<true>, blocks, 256, 0, s, n, b, w.nlc[0], w.nlc[1], w.nlc[2],
-               cellCheck, cutnb2, w.order.as<int>(), w.cellOf.as<int>(), w.cellStart.as<int>(),
-               w.xs.as<double>(), w.ys.as<double>(), w.zs.as<double>(), w.fs.as<int>(),
-               exclStart, exclFlat, w.cnt.as<int>(), w.neighPair.as<int>(),
-               w.off.as<long long>(), w.list.as<int>());
-  } else {
-    w.ncell = 0;
-    MDB_LAUNCH(k_iota, grid_for(n, 256), 256, 0, s, n, w.order.as<int>());
-    const int blocks = grid_for((long long)n * 32, 256);
-    MDB_LAUNCH(k_vl_pairs<false>, blocks, 256, 0, s, n, b, cutnb2, x, y, z, frozen, exclStart,
-               exclFlat, w.cnt.as<int>(), w.neighPair.as<int>(), (const long long *)nullptr,
-               (int *)nullptr);
-    MDB_TRY(exclusive_scan(w.cnt.as<int>(), w.off.as<long long>(), n, w.scanTmp.p, s));
-    long long total = 0;
-    MDB_CUDA(cudaMemcpyAsync(&total, w.off.as<long long>() + n, sizeof(long long),
-                             cudaMemcpyDeviceToHost, s));
-    MDB_CUDA(cudaStreamSynchronize(s));
-    w.entries = total;
-    if (total > 0x7fffffffLL) return MDBAS_NB_ERR_CAPACITY;
-    MDB_TRY(w.list.ensure(sizeof(int) * (size_t)(total > 0 ? total : 1)));
-    MDB_LAUNCH(k_vl_pairs<true>, blocks, 256, 0, s, n, b, cutnb2, x, y, z, frozen, exclStart,
-               exclFlat, w.cnt.as<int>(), w.neighPair.as<int>(), w.off.as<long long>(),
-               w.list.as<int>());
+    MDB_TRY(w.chunkOff.ensure(sizeof(int) * (size_t)ncell * (map.cellCheck + 1)));
   }
-  return MDBAS_NB_OK;
+
+  for (int attempt = 0;; ++attempt) {
+    MDB_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(int), s));
+    float band, lx = 0.f, ly = 0.f, lz = 0.f;
+    int exactOnly = 0;
+    if (linkCells) {
+      int *count = w.cellCount.as<int>(), *fill = count + ncell + 1;
+      MDB_TRY(w.chunkBase.ensure(sizeof(int) * (size_t)ncell * map.stride));
+      map.cellStart = w.cellStart.as<int>();
+      map.cellOf = w.cellOf.as<int>();
+      map.order = w.order.as<int>();
+      map.posOf = w.posOf.as<int>();
+      map.chunkOff = w.chunkOff.as<int>();
+      map.chunkBase = w.chunkBase.as<int>();
+      // coordinates up to two boxes (two roundings), the image shift and
+      // its sum with a coordinate (up to three)
+      const double ext = std::max({fabs(b.a1) + fabs(b.b1) + fabs(b.c1),
+                                   fabs(b.a2) + fabs(b.b2) + fabs(b.c2),
+                                   fabs(b.a3) + fabs(b.b3) + fabs(b.c3)});
+      band = test_band(cutnb, (8. * ext + cutnb) * ulp);
+      MDB_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * 2 * (size_t)(ncell + 1), s));
+      MDB_LAUNCH(k_lc_bin, grid_for(n, 256), 256, 0, s, n, b, w.nlc[0], w.nlc[1], w.nlc[2], x, y,
+                 z, w.xu.as<double>(), w.yu.as<double>(), w.zu.as<double>(), w.cellOf.as<int>(),
+                 count, flags);
+      MDB_TRY(exclusive_scan32(count, w.cellStart.as<int>(), ncell, w.scanTmp.p, s));
+      MDB_LAUNCH(k_lc_scatter, grid_for(n, 256), 256, 0, s, n, w.cellOf.as<int>(),
+                 w.cellStart.as<int>(), fill, w.tmpIdx.as<int>());
+      MDB_LAUNCH(k_lc_order, ncell, 256, 0, s, ncell, w.cellStart.as<int>(), w.tmpIdx.as<int>(),
+                 w.order.as<int>());
+      MDB_LAUNCH(k_lc_gather, grid_for(n, 256), 256, 0, s, ncell, b, w.cellStart.as<int>(),
+                 w.order.as<int>(), w.xu.as<double>(), w.yu.as<double>(), w.zu.as<double>(),
+                 frozen, w.xs.as<double>(), w.ys.as<double>(), w.zs.as<double>(),
+                 w.cs.as<float4>(), w.posOf.as<int>());
+      MDB_LAUNCH(k_lc_chunks, grid_for(ncell, kListWarps), 32 * kListWarps, 0, s, ncell, w.nlc[0],
+                 w.nlc[1], w.nlc[2], map.cellCheck, map.stride, w.cellStart.as<int>(),
+                 w.chunkOff.as<int>(), w.chunkBase.as<int>(), flags, flags + 1);
+    } else {
+      const double bx = b.a1, by = b.type == CUBIC ? b.a1 : b.b2,
+                   bz = b.type == CUBIC ? b.a1 : b.c3;
+      const double ux = b.u1, uy = b.type == CUBIC ? b.u1 : b.v2,
+                   uz = b.type == CUBIC ? b.u1 : b.w3;
+      // the FP32 minimum image is the orthorhombic box's
+      exactOnly = !((b.type == CUBIC || b.type == ORBIC) && bx > 0. && by > 0. && bz > 0. &&
+                    fabs(bx * ux - 1.) < 1e-9 && fabs(by * uy - 1.) < 1e-9 &&
+                    fabs(bz * uz - 1.) < 1e-9);
+      lx = (float)bx;
+      ly = (float)by;
+      lz = (float)bz;
+      // two coordinates of half a box, their difference, the box length and
+      // the difference from it
+      band = test_band(cutnb, 4. * std::max({bx, by, bz}) * ulp);
+      MDB_LAUNCH(k_vl_coords, grid_for(n, 256), 256, 0, s, n, bx, by, bz, x, y, z, frozen,
+                 w.cs.as<float4>(), w.order.as<int>());
+    }
+    long long slab = (long long)(kMaskBytes / (sizeof(unsigned) * (size_t)map.stride)) &
+                     ~(long long)(kGroup - 1);
+    slab = std::max<long long>(slab, kGroup);
+    const bool whole = slab >= n;
+    MDB_TRY(w.masks.ensure(sizeof(unsigned) * (size_t)map.stride * std::min<long long>(slab, n)));
+    const auto test = [&](int p0, int p1) -> int {
+      unsigned *m = w.masks.as<unsigned>();
+      const int g = grid_for(p1 - p0, kGroup * kListWarps);
+      if (linkCells) {
+        const auto kern = frozen ? k_lc_masks<true> : k_lc_masks<false>;
+        MDB_LAUNCH(kern, dim3(g, grid_for(map.stride, kPiece)), 32 * kListWarps, 0, s, p0, p1, b,
+                   map, cutnb2, (float)cutnb2, band, w.xs.as<double>(), w.ys.as<double>(), w.zs.as<double>(), w.cs.as<float4>(),
+                   flags, m);
+      } else {
+        const auto kern = frozen ? k_vl_masks<true> : k_vl_masks<false>;
+        MDB_LAUNCH(kern, dim3(g, grid_for((n + 31) >> 5, kPiece)), 32 * kListWarps, 0, s, p0, p1,
+                   b, map, cutnb2, (float)cutnb2, band, lx, ly, lz, exactOnly, x, y, z,
+                   w.cs.as<float4>(), m);
+      }
+      MDB_LAUNCH(k_list_count, grid_for(p1 - p0, kListWarps), 32 * kListWarps, 0, s, p0, p1, map,
+                 exclStart, exclFlat, flags, m, w.cnt.as<int>(), w.neighPair.as<int>());
+      return MDBAS_NB_OK;
+    };
+    for (long long p = 0; p < n; p += slab) MDB_TRY(test((int)p, (int)std::min<long long>(p + slab, n)));
+    MDB_TRY(exclusive_scan(w.cnt.as<int>(), w.off.as<long long>(), n, w.scanTmp.p, s));
+    struct { long long total; int flags, need; } h;
+    MDB_CUDA(cudaMemcpyAsync(&h, w.off.as<long long>() + n, sizeof(h), cudaMemcpyDeviceToHost, s));
+    MDB_CUDA(cudaStreamSynchronize(s));
+    if (h.flags & FLAG_NONFINITE) return MDBAS_NB_ERR_NONFINITE;
+    if (h.flags & FLAG_OUTSIDE) return MDBAS_NB_ERR_BOX;
+    if (h.flags & FLAG_CELL) {
+      if (attempt > 0) return MDBAS_NB_ERR_CAPACITY;
+      w.maskStride = map.stride = (h.need + 3) & ~3;
+      continue;
+    }
+    w.entries = h.total;
+    if (h.total > 0x7fffffffLL) return MDBAS_NB_ERR_CAPACITY;  // MDBas's int list index
+    MDB_TRY(w.list.ensure(sizeof(int) * (size_t)std::max<long long>(h.total, 1)));
+    for (long long p = 0; p < n; p += slab) {
+      const int p0 = (int)p, p1 = (int)std::min<long long>(p + slab, n);
+      if (!whole) MDB_TRY(test(p0, p1));
+      MDB_LAUNCH(k_list_fill, grid_for(p1 - p0, kListWarps), 32 * kListWarps, 0, s, p0, p1, map,
+                 w.masks.as<unsigned>(), w.off.as<long long>(), w.list.as<int>());
+    }
+    return MDBAS_NB_OK;
+  }
 }
 
 int ref_list_offsets(RefListWork &w, int n, cudaStream_t s) {

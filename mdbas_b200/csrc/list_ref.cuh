@@ -10,14 +10,15 @@ struct RefListWork {
   DBuf list;        // neighList entries (int32)
   DBuf neighPair;   // per atom (int32)
   DBuf order;       // neighOrder (int32)
-  DBuf off;         // entry offset of each neighOrder position (int64, n+1)
+  DBuf off;         // entry offset of each neighOrder position (int64, n+1, then build flags)
   long long entries = 0;
   int linkCells = 0;
   int nlc[3] = {0, 0, 0};
   int ncell = 0;
   // scratch
-  DBuf xu, yu, zu, xs, ys, zs, fs, cellOf, posOf, tmpIdx, cellCount, cellFill, cellStart, cnt,
-      scanTmp, flags;
+  DBuf xu, yu, zu, xs, ys, zs, cs, cellOf, posOf, tmpIdx, cellCount, cellStart, chunkOff,
+      chunkBase, masks, cnt, scanTmp;
+  int maskStride = 0;  // words per mask row of a build denser than estimated
 };
 
 int image_update_device(int n, const DevBox &b, double *x, double *y, double *z, cudaStream_t s);
