@@ -15,6 +15,8 @@
 // the adjoint is the gradient harness's reference-quality path.
 #include "common.cuh"
 #include "engine.cuh"
+#include "pair_rows.cuh"
+#include "real64.cuh"
 
 using namespace mdbas;
 
@@ -78,99 +80,164 @@ __device__ __forceinline__ RadialLJ lj_unit(const PairParams &p, double r, doubl
   return o;
 }
 
+constexpr int kAdjBlocks = 4;  // blocks per SM
+
 struct AdjOut {
   double *gq, *geps, *gsig;   // dE/d(q_i, eps_i, sig_i)
   double *hx, *hy, *hz;       // d(v.F)/dx_i
   double *pq, *peps, *psig;   // d(v.F)/d(q_i, eps_i, sig_i)
 };
 
-__device__ __forceinline__ void adj_pair(const PairParams &p, int i, int j, double dx, double dy,
-                                         double dz, double r2, bool corr, const double *q,
-                                         const double *eps, const double *sig, const double *vx,
-                                         const double *vy, const double *vz, const AdjOut &o,
-                                         double (&acc)[10]) {
+struct RadialPair {
+  RadialQ c;
+  RadialLJ l;
+};
+
+__device__ __noinline__ RadialPair radial_general(const PairParams &p, double r2, double sig) {
+  const double r = sqrt(r2);
+  return RadialPair{ewald_unit(p, r, false), lj_unit(p, r, r2, sig)};
+}
+
+// The same with the forms of real64.cuh (rt = 1/r, x = alpha r in their
+// range, sig an ordinary length or zero).
+__device__ __forceinline__ RadialPair radial_fast(const PairParams &p, double r2, double rt,
+                                                  double r, double x, double sig) {
+  RadialPair o;
+  const double g = expm64(x * x);
+  const double A = p.chargeConst * 2.0 * p.alpha / kSqrtPi;
+  o.c.e = p.chargeConst * (g * erfcx64(x)) * rt;
+  o.c.d1 = -(o.c.e + A * g) * rt;
+  o.c.d2 = -2.0 * o.c.d1 * rt + 2.0 * A * p.alpha * p.alpha * g;
+  o.l = RadialLJ{0., 0., 0., 0., 0.};
+  if (!p.vdwSwitch || sig == 0.) return o;
+  const double t = sig * rt, t2 = t * t;
+  const double s6 = t2 * t2 * t2;
+  const double s12 = s6 * s6;
+  const double isig = rcp64(sig);
+  const double P = 4.0 * (s12 - s6);
+  const double P1 = 24.0 * rt * (s6 - 2.0 * s12);
+  const double P2 = 4.0 * (rt * rt) * (156.0 * s12 - 42.0 * s6);
+  const double Ps = 24.0 * isig * (2.0 * s12 - s6);
+  const double Ps1 = 144.0 * (rt * isig) * (s6 - 4.0 * s12);
+  const bool inner = r2 <= p.cutOn2;
+  const double a = p.cutOff2 - r2, b = p.cutOn2 - r2;
+  const double Su = 6.0 * p.switch2 * a * b;
+  const double Suu = -6.0 * p.switch2 * (p.cutOff2 + p.cutOn2 - 2.0 * r2);
+  const double S =
+      inner ? 1. : a * a * (p.cutOff2 + 2.0 * r2 - 3.0 * p.cutOn2) * p.switch2;
+  const double S1 = inner ? 0. : 2.0 * r * Su;
+  const double S2 = inner ? 0. : 2.0 * Su + 4.0 * r2 * Suu;
+  o.l.g = P * S;
+  o.l.d1 = P1 * S + P * S1;
+  o.l.d2 = P2 * S + 2.0 * P1 * S1 + P * S2;
+  o.l.s = Ps * S;
+  o.l.s1 = Ps1 * S + Ps * S1;
+  return o;
+}
+
+// The pairs within the cut-off: the row walk of pair_rows.cuh, j's sums by
+// FP64 atomics (9 per pair with force weights, 3 without), i's in registers.
+// One thread per atom with the C library's functions took 2.31 ms for 12,000
+// atoms (94 blocks, a serial chain of 347 pairs each); this takes 0.32.
+template <bool HVP>
+__global__ void __launch_bounds__(32 * kRowWarps, kAdjBlocks)
+k_adjoint_pairs(int n, DevBox b, PairParams p, HalfList hl, const double *__restrict__ x,
+                const double *__restrict__ y, const double *__restrict__ z,
+                const double *__restrict__ q, const double *__restrict__ eps,
+                const double *__restrict__ sig, int split, const double *__restrict__ vx,
+                const double *__restrict__ vy, const double *__restrict__ vz, AdjOut o,
+                unsigned *__restrict__ work) {
+  __shared__ RowQueue queues[kRowWarps];
+  const int lane = threadIdx.x & 31;
+  constexpr int N = HVP ? 9 : 3;
+  double qi, ei, si, vxi, vyi, vzi, acc[N];
+  walk_rows(
+      n, split, b, p.cutOff2, hl, x, y, z, queues[threadIdx.x >> 5], work,
+      [&](int i) {
+        qi = q[i];
+        ei = eps[i];
+        si = sig[i];
+        if constexpr (HVP) {
+          vxi = vx[i];
+          vyi = vy[i];
+          vzi = vz[i];
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k) acc[k] = 0.;
+      },
+      [&](int, bool active, int j, double dx, double dy, double dz, double r2) {
+        if (!active) return;
+        const double qj = q[j], ej = eps[j], sg = si + sig[j];
+        const double veps = ei * ej;
+        const double rt = rsqrt64(r2), r = sqrt64(r2, rt), xa = p.alpha * r;
+        const RadialPair f =
+            r2 >= 1e-6 && xa >= 0. && xa <= kErfcxMax && (sg == 0. || (sg >= 1e-3 && sg <= 1e3))
+                ? radial_fast(p, r2, rt, r, xa, sg)
+                : radial_general(p, r2, sg);
+        acc[0] += qj * f.c.e;
+        acc[1] += ej * f.l.g;
+        acc[2] += veps * f.l.s;
+        atomicAdd(o.gq + j, qi * f.c.e);
+        atomicAdd(o.geps + j, ei * f.l.g);
+        atomicAdd(o.gsig + j, veps * f.l.s);
+        if constexpr (HVP) {
+          const double ux = vxi - vx[j], uy = vyi - vy[j], uz = vzi - vz[j];
+          const double ud = (ux * dx + uy * dy + uz * dz) * rt;  // (v_i - v_j).d / r
+          const double qq = qi * qj;
+          const double E1 = qq * f.c.d1 + veps * f.l.d1;
+          const double E2 = qq * f.c.d2 + veps * f.l.d2;
+          const double bb = E1 * rt, a = ud * (E2 - bb) * rt;
+          const double hx = a * dx + bb * ux, hy = a * dy + bb * uy, hz = a * dz + bb * uz;
+          acc[3] -= hx;
+          acc[4] -= hy;
+          acc[5] -= hz;
+          atomicAdd(o.hx + j, hx);
+          atomicAdd(o.hy + j, hy);
+          atomicAdd(o.hz + j, hz);
+          const double cd = f.c.d1 * ud, ld = f.l.d1 * ud, ls = veps * f.l.s1 * ud;
+          acc[6] += qj * cd;
+          acc[7] += ej * ld;
+          acc[8] += ls;
+          atomicAdd(o.pq + j, qi * cd);
+          atomicAdd(o.peps + j, ei * ld);
+          atomicAdd(o.psig + j, ls);
+        }
+      },
+      [&](int i) {
+        double *const dst[9] = {o.gq, o.geps, o.gsig, o.hx, o.hy, o.hz, o.pq, o.peps, o.psig};
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          const double v = warp_sum_d(acc[k]);
+          if (lane == 0) atomicAdd(dst[k] + i, v);
+        }
+      });
+}
+
+// An excluded pair's terms into acc (atom i) and by atomics (atom j).
+__device__ __forceinline__ void adj_excluded(const PairParams &p, int i, int j, double dx,
+                                             double dy, double dz, double r2, const double *q,
+                                             const double *vx, const double *vy,
+                                             const double *vz, const AdjOut &o,
+                                             double (&acc)[5]) {
   const double r = sqrt(r2);
   const double qi = q[i], qj = q[j];
-  const RadialQ c = ewald_unit(p, r, corr);
-  RadialLJ l{0., 0., 0., 0., 0.};
-  double ei = 0., ej = 0., veps = 0.;
-  if (!corr) {
-    ei = eps[i];
-    ej = eps[j];
-    veps = ei * ej;
-    l = lj_unit(p, r, r2, sig[i] + sig[j]);
-  }
-  // dE/d parameters (acc: 0 gq_i, 1 geps_i, 2 gsig_i)
+  const RadialQ c = ewald_unit(p, r, true);
   acc[0] += qj * c.e;
   atomicAdd(o.gq + j, qi * c.e);
-  if (!corr) {
-    acc[1] += ej * l.g;
-    acc[2] += veps * l.s;
-    atomicAdd(o.geps + j, ei * l.g);
-    atomicAdd(o.gsig + j, veps * l.s);
-  }
   if (!vx) return;
   const double ux = vx[i] - vx[j], uy = vy[i] - vy[j], uz = vz[i] - vz[j];
-  const double ud = (ux * dx + uy * dy + uz * dz) / r;  // (v_i - v_j).d / r
-  const double qq = qi * qj;
-  const double E1 = qq * c.d1 + veps * l.d1;
-  const double E2 = qq * c.d2 + veps * l.d2;
+  const double ud = (ux * dx + uy * dy + uz * dz) / r;
+  const double E1 = qi * qj * c.d1, E2 = qi * qj * c.d2;
   const double a = ud * (E2 - E1 / r) / r, b = E1 / r;
   const double hx = a * dx + b * ux, hy = a * dy + b * uy, hz = a * dz + b * uz;
-  acc[3] -= hx;
-  acc[4] -= hy;
-  acc[5] -= hz;
+  acc[1] -= hx;
+  acc[2] -= hy;
+  acc[3] -= hz;
   atomicAdd(o.hx + j, hx);
   atomicAdd(o.hy + j, hy);
   atomicAdd(o.hz + j, hz);
-  // d(v.F)/d parameters (acc: 6 pq_i, 7 peps_i, 8 psig_i)
-  acc[6] += qj * c.d1 * ud;
+  acc[4] += qj * c.d1 * ud;
   atomicAdd(o.pq + j, qi * c.d1 * ud);
-  if (!corr) {
-    acc[7] += ej * l.d1 * ud;
-    acc[8] += veps * l.s1 * ud;
-    atomicAdd(o.peps + j, ei * l.d1 * ud);
-    atomicAdd(o.psig + j, veps * l.s1 * ud);
-  }
-}
-
-__device__ __forceinline__ void adj_flush(int i, const double (&acc)[10], bool hvp,
-                                          const AdjOut &o) {
-  atomicAdd(o.gq + i, acc[0]);
-  atomicAdd(o.geps + i, acc[1]);
-  atomicAdd(o.gsig + i, acc[2]);
-  if (!hvp) return;
-  atomicAdd(o.hx + i, acc[3]);
-  atomicAdd(o.hy + i, acc[4]);
-  atomicAdd(o.hz + i, acc[5]);
-  atomicAdd(o.pq + i, acc[6]);
-  atomicAdd(o.peps + i, acc[7]);
-  atomicAdd(o.psig + i, acc[8]);
-}
-
-// One thread per atom (neighOrder position) over its half-list entries.
-__global__ void __launch_bounds__(128)
-k_adjoint_pairs(int n, DevBox b, PairParams p, const int *__restrict__ order,
-                const int *__restrict__ neighPair, const long long *__restrict__ off,
-                const int *__restrict__ list, const double *__restrict__ x,
-                const double *__restrict__ y, const double *__restrict__ z,
-                const double *__restrict__ q, const double *__restrict__ eps,
-                const double *__restrict__ sig, const double *__restrict__ vx,
-                const double *__restrict__ vy, const double *__restrict__ vz, AdjOut o) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int i = order[t];
-  const long long start = off[t];
-  const int cnt = neighPair[i];
-  double acc[10] = {0., 0., 0., 0., 0., 0., 0., 0., 0., 0.};
-  for (int k = 0; k < cnt; ++k) {
-    const int j = list[start + k];
-    double dx = x[j] - x[i], dy = y[j] - y[i], dz = z[j] - z[i];
-    const double r2 = dist_d(b, dx, dy, dz);
-    if (r2 <= p.cutOff2)
-      adj_pair(p, i, j, dx, dy, dz, r2, false, q, eps, sig, vx, vy, vz, o, acc);
-  }
-  adj_flush(i, acc, vx != nullptr, o);
 }
 
 // Excluded pairs (j > i of each row, no cut-off) and the self term.
@@ -178,12 +245,11 @@ __global__ void __launch_bounds__(128)
 k_adjoint_excl(int n, DevBox b, PairParams p, const int *__restrict__ exclStart,
                const int *__restrict__ exclFlat, const double *__restrict__ x,
                const double *__restrict__ y, const double *__restrict__ z,
-               const double *__restrict__ q, const double *__restrict__ eps,
-               const double *__restrict__ sig, const double *__restrict__ vx,
+               const double *__restrict__ q, const double *__restrict__ vx,
                const double *__restrict__ vy, const double *__restrict__ vz, AdjOut o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double acc[10] = {0., 0., 0., 0., 0., 0., 0., 0., 0., 0.};
+  double acc[5] = {0., 0., 0., 0., 0.};
   acc[0] = -2.0 * p.chargeConst * p.alpha * q[i] / kSqrtPi;  // self term
   const int e = exclStart[i + 1];
   for (int k = exclStart[i]; k < e; ++k) {
@@ -191,9 +257,14 @@ k_adjoint_excl(int n, DevBox b, PairParams p, const int *__restrict__ exclStart,
     if (j <= i) continue;
     double dx = x[j] - x[i], dy = y[j] - y[i], dz = z[j] - z[i];
     const double r2 = dist_d(b, dx, dy, dz);
-    adj_pair(p, i, j, dx, dy, dz, r2, true, q, eps, sig, vx, vy, vz, o, acc);
+    adj_excluded(p, i, j, dx, dy, dz, r2, q, vx, vy, vz, o, acc);
   }
-  adj_flush(i, acc, vx != nullptr, o);
+  atomicAdd(o.gq + i, acc[0]);
+  if (!vx) return;
+  atomicAdd(o.hx + i, acc[1]);
+  atomicAdd(o.hy + i, acc[2]);
+  atomicAdd(o.hz + i, acc[3]);
+  atomicAdd(o.pq + i, acc[4]);
 }
 
 }  // namespace
@@ -214,11 +285,11 @@ extern "C" int mdbas_nb_engine_adjoint(mdbas_nb_engine *e, const double *vx, con
   LaunchScope ls(e);
   const int n = e->n;
   cudaStream_t s = e->stream;
-  // device scratch: 3 (v) + 9 (outputs) arrays of n
-  MDB_TRY(e->adjBuf.ensure(sizeof(double) * 12 * (size_t)n));
+  // device scratch: 3 (v) + 9 (outputs) arrays of n and the work counter
+  MDB_TRY(e->adjBuf.ensure(sizeof(double) * (12 * (size_t)n + 1)));
   double *buf = e->adjBuf.as<double>();
   double *dv = buf, *outs = buf + 3 * (size_t)n;
-  MDB_CUDA(cudaMemsetAsync(outs, 0, sizeof(double) * 9 * (size_t)n, s));
+  MDB_CUDA(cudaMemsetAsync(outs, 0, sizeof(double) * (9 * (size_t)n + 1), s));
   const cudaMemcpyKind in = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const cudaMemcpyKind outk = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   const size_t bytes = sizeof(double) * (size_t)n;
@@ -236,14 +307,17 @@ extern "C" int mdbas_nb_engine_adjoint(mdbas_nb_engine *e, const double *vx, con
   o.pq = ptrs[6]; o.peps = ptrs[7]; o.psig = ptrs[8];
   const double *dvx = hvp ? dv : nullptr, *dvy = hvp ? dv + n : nullptr,
                *dvz = hvp ? dv + 2 * (size_t)n : nullptr;
-  MDB_LAUNCH(k_adjoint_pairs, grid_for(n, 128), 128, 0, s, n, e->box, e->pp,
-             e->ref.order.as<int>(), e->ref.neighPair.as<int>(), e->ref.off.as<long long>(),
-             e->ref.list.as<int>(), e->x.as<double>(), e->y.as<double>(), e->z.as<double>(),
-             e->q.as<double>(), e->eps.as<double>(), e->sig.as<double>(), dvx, dvy, dvz, o);
+  const RowGrid g = row_grid(n, kAdjBlocks);
+  const HalfList hl{e->ref.order.as<int>(), e->ref.neighPair.as<int>(),
+                    e->ref.off.as<long long>(), e->ref.list.as<int>()};
+  const auto kern = hvp ? k_adjoint_pairs<true> : k_adjoint_pairs<false>;
+  MDB_LAUNCH(kern, g.blocks, 32 * kRowWarps, 0, s, n, e->box, e->pp, hl, e->x.as<double>(),
+             e->y.as<double>(), e->z.as<double>(), e->q.as<double>(), e->eps.as<double>(),
+             e->sig.as<double>(), g.split, dvx, dvy, dvz, o,
+             reinterpret_cast<unsigned *>(outs + 9 * (size_t)n));
   MDB_LAUNCH(k_adjoint_excl, grid_for(n, 128), 128, 0, s, n, e->box, e->pp,
              e->exclStart.as<int>(), e->exclFlat.as<int>(), e->x.as<double>(),
-             e->y.as<double>(), e->z.as<double>(), e->q.as<double>(), e->eps.as<double>(),
-             e->sig.as<double>(), dvx, dvy, dvz, o);
+             e->y.as<double>(), e->z.as<double>(), e->q.as<double>(), dvx, dvy, dvz, o);
   double *dst[9] = {gq, geps, gsig, hx, hy, hz, pq, peps, psig};
   for (int k = 0; k < (hvp ? 9 : 3); ++k)
     MDB_CUDA(cudaMemcpyAsync(dst[k], ptrs[k], bytes, outk, s));

@@ -14,10 +14,9 @@
 // real64.cuh (a few ulp from the C library's; the forces of a 3,000-atom
 // water box are 1.98e-15 from a long-double sum, 2.15e-15 with the C
 // library's).  The order of the FP64 additions is not fixed.
-#include <algorithm>
-
 #include "common.cuh"
 #include "pair_fp64.cuh"
+#include "pair_rows.cuh"
 #include "real64.cuh"
 
 namespace mdbas {
@@ -178,56 +177,28 @@ __device__ __forceinline__ PairTerms pair_ewald_fast(const PairParams &p, const 
 // Smallest r2 of the fast form: far below any atomic distance, far above
 // where its powers of 1/r could overflow.
 constexpr double kFastR2Min = 1e-6;
-constexpr int kPairWarps = 4;     // warps per block
-constexpr int kPairQueue = 64;    // queued pairs per warp
 constexpr int kPairBlocks = 6;    // blocks per SM
-
-// dist() of a pair whose displacement lies within half a box (times the
-// margin) along every axis needs no image: nint() is 0 there and MDBas
-// subtracts an exact zero.  The bound is compared on the high words.
-__device__ __forceinline__ bool near_d(int hx, int hy, int hz, double dx, double dy, double dz) {
-  return (__double2hiint(dx) & 0x7fffffff) < hx && (__double2hiint(dy) & 0x7fffffff) < hy &&
-         (__double2hiint(dz) & 0x7fffffff) < hz;
-}
 
 // acc[0..4]: elec, vdw, virelec, virvdw, in-cut-off pairs; acc[7]: the work
 // counter.
 //
-// One warp per atom i, lanes over i's list entries (a coalesced read); the
-// entries inside the cut-off are queued in shared memory and evaluated 32 at
-// a time, so the FP64 arithmetic runs with full warps (62% of a 14 A list
-// lies within 12 A).  Bound by latency and the LSU (gathers and scattered
-// additions, 60% of the data-pipe cycles; FP64 pipe 40%): entries are loaded
-// two rounds ahead and positions one round ahead (0.93 -> 0.67 ms).  Measured
-// against one thread per atom with the C library's functions: 2.26 -> 0.67 ms
-// at 96,000 atoms of water, 1.22 -> 0.10 at 12,000, 1.23 -> 0.046 at 3,000.
+// The row walk of pair_rows.cuh; warps keep their energy sums in registers
+// over all their atoms.  Bound by latency and the LSU (gathers and scattered
+// additions, 60% of the data-pipe cycles; FP64 pipe 40%).  Measured against
+// one thread per atom with the C library's functions: 2.26 -> 0.67 ms at
+// 96,000 atoms of water, 1.22 -> 0.10 at 12,000, 1.23 -> 0.046 at 3,000.
 // Atoms packed to one 32-byte sector and j forces added a sector at a time
-// measured no better (0.67 and 1.1 ms).  Warps keep their energy sums in registers over all
-// their atoms.
-//
-// An atom's row is cut into 2^split work items, so that a small system fills
-// the SMs.
+// measured no better (0.67 and 1.1 ms).
 template <bool EWALD>
-__global__ void __launch_bounds__(32 * kPairWarps, kPairBlocks)
-k_pairs_fp64(int n, DevBox b, PairParams p, const int *__restrict__ order,
-             const int *__restrict__ neighPair, const long long *__restrict__ off,
-             const int *__restrict__ list, const double *__restrict__ x,
+__global__ void __launch_bounds__(32 * kRowWarps, kPairBlocks)
+k_pairs_fp64(int n, DevBox b, PairParams p, HalfList hl, const double *__restrict__ x,
              const double *__restrict__ y, const double *__restrict__ z,
              const double *__restrict__ q, const double *__restrict__ eps,
              const double *__restrict__ sig, int split, double *__restrict__ fx,
              double *__restrict__ fy, double *__restrict__ fz, double *__restrict__ acc) {
-  __shared__ double sq[kPairWarps][4][kPairQueue];
-  __shared__ int sj[kPairWarps][kPairQueue];
-  __shared__ double red[5][kPairWarps];
+  __shared__ RowQueue queues[kRowWarps];
+  __shared__ double red[5][kRowWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double (*const qd)[kPairQueue] = sq[w];
-  int *const qj = sj[w];
-  const unsigned lt = (1u << lane) - 1u;
-  // nint() is 0 below 0.499 box lengths (orthorhombic axes; 0: always dist())
-  const bool ortho = b.type == CUBIC || b.type == ORBIC;
-  const int hx = ortho ? __double2hiint(0.499 / fabs(b.u1)) : 0;
-  const int hy = ortho ? __double2hiint(0.499 / fabs(b.type == CUBIC ? b.u1 : b.v2)) : 0;
-  const int hz = ortho ? __double2hiint(0.499 / fabs(b.type == CUBIC ? b.u1 : b.w3)) : 0;
   EwaldConst ek;
   ek.g0 = 2.0 * p.alpha / kSqrtPi;
   ek.a2 = p.alpha * p.alpha;
@@ -236,111 +207,51 @@ k_pairs_fp64(int n, DevBox b, PairParams p, const int *__restrict__ order,
   ek.swc = p.cutOff2 - 3. * p.cutOn2;
   double eel = 0., evdw = 0., virel = 0., virvdw = 0.;
   int npair = 0;
-  // atoms are handed out by a counter (acc[7], zero on entry), the next one
-  // fetched while the current one runs
-  unsigned *const work = reinterpret_cast<unsigned *>(acc + 7);
-  unsigned next = 0;
-  if (lane == 0) next = atomicAdd(work, 1u);
-  for (;;) {
-    const unsigned t = __shfl_sync(0xffffffffu, next, 0);
-    if (t >= (unsigned)n << split) break;
-    if (lane == 0) next = atomicAdd(work, 1u);
-    const unsigned at = t >> split;
-    const int i = order[at];
-    // this item's share of the row, in whole rounds of 32
-    const long long all = neighPair[i];
-    const unsigned part = t & ((1u << split) - 1u);
-    const int first = (int)((all * part) >> split) & ~31;
-    const int cnt = (part + 1 == 1u << split ? (int)all : (int)((all * (part + 1)) >> split) & ~31) -
-                    first;
-    const int *row = list + off[at] + first;
-    const double xi = x[i], yi = y[i], zi = z[i], ei = eps[i], si = sig[i];
-    const double qi = EWALD ? p.chargeConst * q[i] : q[i];
-    double fxi = 0., fyi = 0., fzi = 0.;
-    // entries two rounds ahead, their positions one round ahead
-    int jc = lane < cnt ? row[lane] : -1;
-    int jn = 32 + lane < cnt ? row[32 + lane] : -1;
-    double px = 0., py = 0., pz = 0.;
-    const auto fetch = [&](int j) {
-      if (j >= 0) {
-        px = x[j];
-        py = y[j];
-        pz = z[j];
-      }
-    };
-    fetch(jc);
-    int qn = 0, k = 0;
-    while (k < cnt || qn > 0) {
-      while (k < cnt && qn < 32) {
-        const int j = jc;
-        double dx = px - xi, dy = py - yi, dz = pz - zi;
-        k += 32;
-        jc = jn;
-        fetch(jc);
-        jn = k + 32 + lane < cnt ? row[k + 32 + lane] : -1;
-        const double r2 = near_d(hx, hy, hz, dx, dy, dz)
-                              ? dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz))
-                              : dist_d(b, dx, dy, dz);
-        const bool in = j >= 0 && r2 <= p.cutOff2;
-        const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (in) {
-          const int o = qn + __popc(m & lt);
-          qd[0][o] = dx;
-          qd[1][o] = dy;
-          qd[2][o] = dz;
-          qd[3][o] = r2;
-          qj[o] = j;
-        }
-        qn += __popc(m);
-      }
-      __syncwarp();
-      const int take = min(qn, 32);
-      qn -= take;
-      npair += take;
-      double fxj = 0., fyj = 0., fzj = 0.;
-      int j = 0;
-      if (lane < take) {
-        const int o = qn + lane;
-        const double dx = qd[0][o], dy = qd[1][o], dz = qd[2][o], r2 = qd[3][o];
-        j = qj[o];
+  double qi, ei, si, fxi, fyi, fzi;
+  walk_rows(
+      n, split, b, p.cutOff2, hl, x, y, z, queues[w], reinterpret_cast<unsigned *>(acc + 7),
+      [&](int i) {
+        qi = EWALD ? p.chargeConst * q[i] : q[i];
+        ei = eps[i];
+        si = sig[i];
+        fxi = fyi = fzi = 0.;
+      },
+      [&](int take, bool active, int j, double dx, double dy, double dz, double r2) {
+        npair += take;
+        if (!active) return;
         const double qq = qi * q[j], veps = ei * eps[j], vsig = si + sig[j];
-        PairTerms o2;
+        PairTerms o;
         if constexpr (EWALD) {
           const double rt = rsqrt64(r2);
           const double xa = p.alpha * sqrt64(r2, rt);
           if (r2 >= kFastR2Min && xa >= 0. && xa <= kErfcxMax)
-            o2 = pair_ewald_fast(p, ek, qq, veps, vsig, r2, rt, xa);
+            o = pair_ewald_fast(p, ek, qq, veps, vsig, r2, rt, xa);
           else
-            o2 = pair_ewald_slow(p, qq, veps, vsig, r2);
+            o = pair_ewald_slow(p, qq, veps, vsig, r2);
         } else {
-          o2 = pair_general<false>(p, qq, veps, vsig, r2);
+          o = pair_general<false>(p, qq, veps, vsig, r2);
         }
-        eel += o2.eel;
-        evdw += o2.evdw;
-        virel += o2.wel;
-        virvdw += o2.wvdw;
-        fxj = o2.f * dx;
-        fyj = o2.f * dy;
-        fzj = o2.f * dz;
+        eel += o.eel;
+        evdw += o.evdw;
+        virel += o.wel;
+        virvdw += o.wvdw;
+        const double fxj = o.f * dx, fyj = o.f * dy, fzj = o.f * dz;
         fxi += fxj;
         fyi += fyj;
         fzi += fzj;
-      }
-      if (lane < take) {
         atomicAdd(fx + j, -fxj);
         atomicAdd(fy + j, -fyj);
         atomicAdd(fz + j, -fzj);
-      }
-      __syncwarp();  // the queue is read before the next round writes
-    }
-    fxi = warp_sum_d(fxi);
-    fyi = warp_sum_d(fyi);
-    fzi = warp_sum_d(fzi);
-    if (lane < 3) {
-      const double v = lane == 0 ? fxi : lane == 1 ? fyi : fzi;
-      atomicAdd((lane == 0 ? fx : lane == 1 ? fy : fz) + i, v);
-    }
-  }
+      },
+      [&](int i) {
+        fxi = warp_sum_d(fxi);
+        fyi = warp_sum_d(fyi);
+        fzi = warp_sum_d(fzi);
+        if (lane < 3) {
+          const double v = lane == 0 ? fxi : lane == 1 ? fyi : fzi;
+          atomicAdd((lane == 0 ? fx : lane == 1 ? fy : fz) + i, v);
+        }
+      });
   const double sum[4] = {warp_sum_d(eel), warp_sum_d(evdw), warp_sum_d(virel),
                          warp_sum_d(virvdw)};
   if (lane == 0) {
@@ -350,7 +261,7 @@ k_pairs_fp64(int n, DevBox b, PairParams p, const int *__restrict__ order,
   __syncthreads();
   if (threadIdx.x < 5) {
     double v = 0.;
-    for (int c = 0; c < kPairWarps; ++c) v += red[threadIdx.x][c];
+    for (int c = 0; c < kRowWarps; ++c) v += red[threadIdx.x][c];
     atomicAdd(acc + threadIdx.x, v);
   }
 }
@@ -541,17 +452,11 @@ int pairs_fp64(int ewald, int n, const DevBox &b, const PairParams &p, const int
                const double *sig, double *fx, double *fy, double *fz, double *acc,
                cudaStream_t s) {
   if (n <= 0) return MDBAS_NB_OK;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = sms * kPairBlocks, warps = grid * kPairWarps;
-  // fewer than two atoms per resident warp: rows cut in two (3,000 atoms 52 ->
-  // 40 us, 6,000 65 -> 62; 12,000 100 -> 106, so not beyond)
-  const int split = n < 2 * warps ? 1 : 0;
+  const RowGrid g = row_grid(n, kPairBlocks);
+  const HalfList hl{order, neighPair, off, list};
   const auto kern = ewald ? k_pairs_fp64<true> : k_pairs_fp64<false>;
-  MDB_LAUNCH(kern, std::min(grid_for((long long)n << split, kPairWarps), grid), 32 * kPairWarps, 0,
-             s, n, b, p, order, neighPair, off, list, x, y, z, q, eps, sig, split, fx, fy, fz,
-             acc);
+  MDB_LAUNCH(kern, g.blocks, 32 * kRowWarps, 0, s, n, b, p, hl, x, y, z, q, eps, sig, g.split, fx,
+             fy, fz, acc);
   return MDBAS_NB_OK;
 }
 
