@@ -8,18 +8,19 @@
 //
 //   * the k list (and e^{-k^2/4a^2}/k^2, the virial factor) is built on the
 //     host with MDBas's expressions and cached per box, alpha and m-range;
+//   * k_ewald_tables: the atoms' cos/sin tables, by MDBas's recurrence, once;
 //   * k_ewald_sf: one thread per k-vector sums q_i e^{i k.r_i} over a range
-//     of atoms; a tile of atoms at a time has its cos/sin tables built in
-//     shared memory with MDBas's recurrence; partial sums per atom range are
-//     added in a fixed order by k_ewald_kdata (deterministic);
-//   * k_ewald_forces: one thread per atom walks the k list in MDBas's order
-//     (rows of fixed (m1, m2), m3 contiguous), so each force component is
-//     accumulated in MDBas's order; its m3 table sits in shared memory.
+//     of atoms, a tile of their tables at a time in shared memory; partial
+//     sums per atom range are added in a fixed order by k_ewald_kdata
+//     (deterministic);
+//   * k_ewald_forces: one thread per atom and part of the k list (rows of
+//     fixed (m1, m2), m3 contiguous); a row's terms share the vector of its
+//     first two indices, so per k only the two sums over m3 are needed;
+//   * k_ewald_add: the parts added in order, scaled, into the forces.
 //
-// This file is compiled with --fmad=false: the table recurrences and the
-// per-(atom, k) products are MDBas's operations; only cos/sin of the first
-// table entry (CUDA's vs the host's) and the order of the sums over atoms
-// differ.
+// This file is compiled with --fmad=false (the table recurrences are MDBas's
+// operations); products and sums over k and atoms use FMAs and an order of
+// their own.
 #include <math.h>
 #include <string.h>
 
@@ -33,6 +34,7 @@ namespace {
 constexpr double kTwoPi = 6.283185307179586;  // include/global.h:54
 constexpr double kPi = 3.141592653589793;
 constexpr int kSfThreads = 256;               // k-vectors per structure-factor block
+constexpr int kEwParts = 32;                  // most parts of the force kernel's k list
 
 struct EwBox {
   double u1, u2, u3, v1, v2, v3, w1, w2, w3;
@@ -65,16 +67,31 @@ __device__ __forceinline__ void ew_table(double s, int M, double *c, double *sn,
   }
 }
 
+// The tables of all atoms, entry e of atom i at tab[e n + i]; entries in the
+// order cos(m s1), sin(m s1), m = 0..M1, then dimension 2 and 3.  One thread
+// per atom and dimension (grid y).
+__global__ void __launch_bounds__(128)
+    k_ewald_tables(int n, EwBox b, int M1, int M2, int M3, const double *__restrict__ x,
+                   const double *__restrict__ y, const double *__restrict__ z,
+                   double *__restrict__ tab) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int d = blockIdx.y;
+  const int M = d == 0 ? M1 : d == 1 ? M2 : M3;
+  const int e = d == 0 ? 0 : d == 1 ? 2 * (M1 + 1) : 2 * (M1 + M2 + 2);
+  double *c = tab + (size_t)e * n + i;
+  ew_table(frac_s(b, d, x[i], y[i], z[i]), M, c, c + (size_t)(M + 1) * n, n);
+}
+
 // Structure factors: part[(2p) K + k], part[(2p+1) K + k] = sum over the atoms
 // of range p of q_i cos(k.r_i), q_i sin(k.r_i).
 __global__ void __launch_bounds__(kSfThreads)
-    k_ewald_sf(int n, int K, int perPart, int tile, EwBox b, int M1, int M2, int M3,
-               const int4 *__restrict__ km, const double *__restrict__ x,
-               const double *__restrict__ y, const double *__restrict__ z,
+    k_ewald_sf(int n, int K, int perPart, int tile, int M1, int M2, int M3,
+               const int4 *__restrict__ km, const double *__restrict__ tab,
                const double *__restrict__ q, double *__restrict__ part) {
   extern __shared__ double sh[];
   const int W = 2 * (M1 + M2 + M3 + 3);  // doubles per atom
-  double *qs = sh + (size_t)tile * W;
+  const int st = W | 1;                  // odd stride: no bank conflicts on the way in
   const int o1s = M1 + 1, o2c = 2 * (M1 + 1), o2s = o2c + M2 + 1, o3c = o2s + M2 + 1,
             o3s = o3c + M3 + 1;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -94,31 +111,24 @@ __global__ void __launch_bounds__(kSfThreads)
   for (int t0 = a0; t0 < a1; t0 += tile) {
     const int na = min(tile, a1 - t0);
     __syncthreads();
-    for (int task = threadIdx.x; task < 3 * na; task += blockDim.x) {
-      const int a = task / 3, d = task - 3 * a, i = t0 + a;
-      const double s = frac_s(b, d, x[i], y[i], z[i]);
-      double *base = sh + (size_t)a * W;
-      if (d == 0) {
-        ew_table(s, M1, base, base + o1s, 1);
-        qs[a] = q[i];
-      } else if (d == 1) {
-        ew_table(s, M2, base + o2c, base + o2s, 1);
-      } else {
-        ew_table(s, M3, base + o3c, base + o3s, 1);
-      }
+    for (int v = threadIdx.x; v < na * W; v += blockDim.x) {
+      const int e = v / na, a = v - e * na;
+      const double c = tab[(size_t)e * n + t0 + a];
+      // the charge goes with the first dimension's entries
+      sh[a * st + e] = e < o2c ? q[t0 + a] * c : c;
     }
     __syncthreads();
     if (k < K) {
+#pragma unroll 2
       for (int a = 0; a < na; ++a) {
-        const double *base = sh + (size_t)a * W;
+        const double *base = sh + (size_t)a * st;
         const double c1 = base[m1], s1 = base[o1s + m1];
         const double c2 = base[o2c + am2], s2 = sg2 * base[o2s + am2];
         const double c3 = base[o3c + am3], s3 = sg3 * base[o3s + am3];
-        const double cm = c1 * c2 - s1 * s2;
-        const double smv = s1 * c2 + c1 * s2;
-        const double qa = qs[a];
-        sc += qa * (cm * c3 - smv * s3);
-        ss += qa * (smv * c3 + cm * s3);
+        const double cm = fma(c1, c2, -(s1 * s2));
+        const double smv = fma(s1, c2, c1 * s2);
+        sc = fma(-smv, s3, fma(cm, c3, sc));
+        ss = fma(cm, s3, fma(smv, c3, ss));
       }
     }
   }
@@ -129,11 +139,14 @@ __global__ void __launch_bounds__(kSfThreads)
 }
 
 // Per k: the structure factor (range sums in order), its energy term and
-// virial/stress terms (src/ewald.c:300-318); block partials of
-// {energy, stress 0..5} into bpart[q * gridDim.x + block].
+// virial/stress terms (src/ewald.c:300-318); S receives it times a_k, as the
+// forces take it.  Block partials of {energy, stress 0..5} go to
+// bpart[q * gridDim.x + block]; the last block to finish adds them, block by
+// block, into sums (*done counts the blocks and returns to 0).
 __global__ void k_ewald_kdata(int K, int P, const double *__restrict__ part,
                               const double4 *__restrict__ kv, const double *__restrict__ vam,
-                              double2 *__restrict__ S, double *__restrict__ bpart) {
+                              double2 *__restrict__ S, double *bpart, unsigned *done,
+                              double *__restrict__ sums) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   double v[7] = {0., 0., 0., 0., 0., 0., 0.};
   if (k < K) {
@@ -142,8 +155,8 @@ __global__ void k_ewald_kdata(int K, int P, const double *__restrict__ part,
       sc += part[(size_t)(2 * p) * K + k];
       ss += part[(size_t)(2 * p + 1) * K + k];
     }
-    S[k] = make_double2(sc, ss);
     const double4 t = kv[k];
+    S[k] = make_double2(t.w * sc, t.w * ss);
     double virtmp = sc * sc + ss * ss;
     v[0] = t.w * virtmp;
     virtmp *= vam[k];
@@ -166,86 +179,93 @@ __global__ void k_ewald_kdata(int K, int P, const double *__restrict__ part,
     double s = 0.;
     for (int j = 0; j < (int)(blockDim.x >> 5); ++j) s += red[threadIdx.x][j];
     bpart[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
+    __threadfence();
   }
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || w >= 7) return;
+  __threadfence();
+  double s = 0.;
+  for (int b = lane; b < (int)gridDim.x; b += 32)
+    s += __ldcg(bpart + (size_t)w * gridDim.x + b);
+  s = warp_sum_d(s);
+  if (lane == 0) sums[w] = s;
 }
 
-__global__ void k_ewald_finish(int nPart, const double *__restrict__ bpart,
-                               double *__restrict__ sums) {
-  __shared__ double red[8];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int j = 0; j < 7; ++j) {
-    double s = 0.;
-    for (int b = threadIdx.x; b < nPart; b += blockDim.x) s += bpart[(size_t)j * nPart + b];
-    s = warp_sum_d(s);
-    if (lane == 0) red[w] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-      sums[j] = t;
-    }
-    __syncthreads();
-  }
-}
-
-// Forces: one thread per atom walks the rows in MDBas's order.  scaleInput:
-// MDBas's ewald_rec multiplies the whole force arrays by fact0 at the end
-// (src/ewald.c:335-340), f = fact0 (f_in + sum); otherwise f = f_in +
-// fact0 sum.  t12: the atom's m1 and m2 tables, SoA [m][n] scratch.
-__global__ void k_ewald_forces(int n, EwBox b, int M1, int M2, int M3, int nRows,
-                               const int4 *__restrict__ rows, const int *__restrict__ rowK,
-                               const double4 *__restrict__ kv, const double2 *__restrict__ S,
-                               const double *__restrict__ x, const double *__restrict__ y,
-                               const double *__restrict__ z, const double *__restrict__ q,
-                               double *__restrict__ t12, double fact0, int scaleInput,
-                               double *__restrict__ fx, double *__restrict__ fy,
-                               double *__restrict__ fz) {
+// Forces: one thread per atom and part of the k list (grid y): pf[3 part + c]
+// [i] = q_i sum over the part's k of a_k (sin(k.r) Re S - cos(k.r) Im S) k_c.
+// Along a row of fixed (m1, m2), k = base + m3 w, so the row adds base sum(d)
+// + w sum(m3 d): eleven FP64 operations per k where the three components took
+// eighteen.  The parts fill the SMs: one thread over the whole list was 24
+// blocks for 3,000 atoms and took 0.99 ms; in 32 parts it takes 0.029.
+__global__ void __launch_bounds__(128)
+    k_ewald_forces(int n, int M1, int M2, int M3, int step, const int *__restrict__ rowPart,
+                   const int4 *__restrict__ rows, const int *__restrict__ rowK,
+                   const double4 *__restrict__ rowBase, double wx, double wy, double wz,
+                   const double2 *__restrict__ S, const double *__restrict__ tab,
+                   const double *__restrict__ q, double *__restrict__ pf) {
   extern __shared__ double sh[];
   const int T = blockDim.x;
-  double *c3 = sh, *s3 = sh + (size_t)(M3 + 1) * T;
+  double *c3 = sh + threadIdx.x, *s3 = c3 + (size_t)(M3 + 1) * T;
   const int i = blockIdx.x * T + threadIdx.x;
   if (i >= n) return;  // no block-wide synchronisation below
-  const double xi = x[i], yi = y[i], zi = z[i], qi = q[i];
-  double *c1 = t12, *s1 = c1 + (size_t)(M1 + 1) * n;
-  double *c2 = s1 + (size_t)(M1 + 1) * n, *s2 = c2 + (size_t)(M2 + 1) * n;
-  ew_table(frac_s(b, 0, xi, yi, zi), M1, c1 + i, s1 + i, n);
-  ew_table(frac_s(b, 1, xi, yi, zi), M2, c2 + i, s2 + i, n);
-  ew_table(frac_s(b, 2, xi, yi, zi), M3, c3 + threadIdx.x, s3 + threadIdx.x, T);
-  double ax = fx[i], ay = fy[i], az = fz[i];
-  if (!scaleInput) ax = ay = az = 0.;
-  for (int r = 0; r < nRows; ++r) {
+  const double *c1 = tab + i, *s1 = c1 + (size_t)(M1 + 1) * n;
+  const double *c2 = s1 + (size_t)(M1 + 1) * n, *s2 = c2 + (size_t)(M2 + 1) * n;
+  const double *c3g = s2 + (size_t)(M2 + 1) * n, *s3g = c3g + (size_t)(M3 + 1) * n;
+  for (int m = 0; m <= M3; ++m) {
+    c3[m * T] = c3g[(size_t)m * n];
+    s3[m * T] = s3g[(size_t)m * n];
+  }
+  double ax = 0., ay = 0., az = 0.;
+  const int r1 = rowPart[(blockIdx.y + 1) * step];
+  for (int r = rowPart[blockIdx.y * step]; r < r1; ++r) {
     const int4 row = rows[r];  // m1, m2, first m3, last m3
     const int am2 = abs(row.y);
-    const double sg2 = row.y < 0 ? -1. : 1.;
-    const double a1c = c1[(size_t)row.x * n + i], a1s = s1[(size_t)row.x * n + i];
-    const double a2c = c2[(size_t)am2 * n + i], a2s = sg2 * s2[(size_t)am2 * n + i];
-    const double cm = a1c * a2c - a1s * a2s;
-    const double smv = a1s * a2c + a1c * a2s;
-    int k = rowK[r];
-    for (int m3 = row.z; m3 <= row.w; ++m3, ++k) {
-      const int am3 = abs(m3);
-      const double sg3 = m3 < 0 ? -1. : 1.;
-      const double t3c = c3[(size_t)am3 * T + threadIdx.x];
-      const double t3s = sg3 * s3[(size_t)am3 * T + threadIdx.x];
-      const double cms = qi * (cm * t3c - smv * t3s);
-      const double sms = qi * (smv * t3c + cm * t3s);
-      const double4 kk = kv[k];
-      const double2 sk = S[k];
-      const double de = kk.w * (sms * sk.x - cms * sk.y);
-      ax += kk.x * de;
-      ay += kk.y * de;
-      az += kk.z * de;
+    const double a1c = c1[(size_t)row.x * n], a1s = s1[(size_t)row.x * n];
+    const double a2c = c2[(size_t)am2 * n];
+    const double a2s = (row.y < 0 ? -1. : 1.) * s2[(size_t)am2 * n];
+    const double cm = fma(a1c, a2c, -(a1s * a2s));
+    const double smv = fma(a1s, a2c, a1c * a2s);
+    const double2 *sk = S + rowK[r] - row.z;
+    double A = 0., B = 0.;
+#pragma unroll 4
+    for (int m3 = row.z; m3 <= row.w; ++m3) {
+      const int at = abs(m3) * T;
+      const double t3c = c3[at], t3s = m3 < 0 ? -s3[at] : s3[at];
+      const double cms = fma(cm, t3c, -(smv * t3s));
+      const double sms = fma(smv, t3c, cm * t3s);
+      const double2 f = sk[m3];
+      const double de = fma(sms, f.x, -(cms * f.y));
+      A += de;
+      B = fma((double)m3, de, B);
     }
+    const double4 base = rowBase[r];
+    ax = fma(B, wx, fma(A, base.x, ax));
+    ay = fma(B, wy, fma(A, base.y, ay));
+    az = fma(B, wz, fma(A, base.z, az));
   }
-  if (scaleInput) {
-    fx[i] = ax * fact0;
-    fy[i] = ay * fact0;
-    fz[i] = az * fact0;
-  } else {
-    fx[i] += ax * fact0;
-    fy[i] += ay * fact0;
-    fz[i] += az * fact0;
-  }
+  const double qi = q[i];
+  double *o = pf + (size_t)3 * blockIdx.y * n + i;
+  o[0] = qi * ax;
+  o[n] = qi * ay;
+  o[2 * (size_t)n] = qi * az;
+}
+
+// The parts in order into the forces (grid y: the component).  scaleInput:
+// MDBas's ewald_rec multiplies the whole force arrays by fact0 at the end
+// (src/ewald.c:335-340), f = fact0 (f_in + sum); otherwise f = f_in + fact0
+// sum.
+__global__ void k_ewald_add(int n, int parts, const double *__restrict__ pf, double fact0,
+                            int scaleInput, double *__restrict__ fx, double *__restrict__ fy,
+                            double *__restrict__ fz) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double *f = (blockIdx.y == 0 ? fx : blockIdx.y == 1 ? fy : fz) + i;
+  double s = 0.;
+  for (int p = 0; p < parts; ++p) s += pf[((size_t)3 * p + blockIdx.y) * n + i];
+  *f = scaleInput ? (*f + s) * fact0 : *f + s * fact0;
 }
 
 // The standalone calls' state (the engine keeps its own).
@@ -268,7 +288,7 @@ int build_klist(EwaldKList &kl, const PBC *box, double alpha, int M1, int M2, in
   rc = rc * 1.05 * kTwoPi;
   const double rc2 = rc * rc;
   std::vector<int4> km, rows;
-  std::vector<double4> kv;
+  std::vector<double4> kv, rowBase;
   std::vector<double> vam;
   std::vector<int> rowK;
   int m2min = 0, m3min = 1;
@@ -292,6 +312,7 @@ int build_klist(EwaldKList &kl, const PBC *box, double alpha, int M1, int M2, in
           if (open && m3 != last + 1) {
             rows.push_back(make_int4(m1, m2, lo, last));
             rowK.push_back((int)km.size() - (last - lo + 1));
+            rowBase.push_back(make_double4(rm2x, rm2y, rm2z, 0.));
             open = false;
           }
           if (!open) {
@@ -309,10 +330,17 @@ int build_klist(EwaldKList &kl, const PBC *box, double alpha, int M1, int M2, in
       if (open) {
         rows.push_back(make_int4(m1, m2, lo, last));
         rowK.push_back((int)km.size() - (last - lo + 1));
+        rowBase.push_back(make_double4(rm2x, rm2y, rm2z, 0.));
       }
       m3min = -M3;
     }
     m2min = -M2;
+  }
+  // first row of each of kEwParts parts of about equally many k
+  int rowPart[kEwParts + 1];
+  for (int p = 0, r = 0; p <= kEwParts; ++p) {
+    while (r < (int)rows.size() && (long long)rowK[r] * kEwParts < (long long)km.size() * p) ++r;
+    rowPart[p] = p == kEwParts ? (int)rows.size() : r;
   }
   kl.K = (int)km.size();
   kl.nRows = (int)rows.size();
@@ -325,6 +353,9 @@ int build_klist(EwaldKList &kl, const PBC *box, double alpha, int M1, int M2, in
   MDB_TRY(kl.vam.ensure(sizeof(double) * K1));
   MDB_TRY(kl.rows.ensure(sizeof(int4) * R1));
   MDB_TRY(kl.rowK.ensure(sizeof(int) * R1));
+  MDB_TRY(kl.rowBase.ensure(sizeof(double4) * R1));
+  MDB_TRY(kl.rowPart.ensure(sizeof(rowPart)));
+  MDB_CUDA(cudaMemcpy(kl.rowPart.p, rowPart, sizeof(rowPart), cudaMemcpyHostToDevice));
   if (kl.K) {
     MDB_CUDA(cudaMemcpy(kl.km.p, km.data(), sizeof(int4) * km.size(), cudaMemcpyHostToDevice));
     MDB_CUDA(cudaMemcpy(kl.kv.p, kv.data(), sizeof(double4) * kv.size(), cudaMemcpyHostToDevice));
@@ -333,6 +364,8 @@ int build_klist(EwaldKList &kl, const PBC *box, double alpha, int M1, int M2, in
     MDB_CUDA(cudaMemcpy(kl.rows.p, rows.data(), sizeof(int4) * rows.size(),
                         cudaMemcpyHostToDevice));
     MDB_CUDA(cudaMemcpy(kl.rowK.p, rowK.data(), sizeof(int) * rowK.size(),
+                        cudaMemcpyHostToDevice));
+    MDB_CUDA(cudaMemcpy(kl.rowBase.p, rowBase.data(), sizeof(double4) * rowBase.size(),
                         cudaMemcpyHostToDevice));
   }
   memcpy(kl.key, key, sizeof(key));
@@ -365,7 +398,7 @@ int ewald_launch_impl(EwaldWork &c, int n, const PBC *box, double alpha, double 
   // shared memory: the k-thread kernel's atom tile, the atom kernel's m3 table
   int maxSmem = 0;
   MDB_CUDA(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t perAtom = sizeof(double) * (2 * (size_t)(M1 + M2 + M3 + 3) + 1);
+  const size_t perAtom = sizeof(double) * (2 * (size_t)(M1 + M2 + M3 + 3) | 1);
   int tile = (int)((size_t)(maxSmem / 2) / perAtom);
   if (tile > 64) tile = 64;
   int fThreads = 128;
@@ -376,14 +409,21 @@ int ewald_launch_impl(EwaldWork &c, int n, const PBC *box, double alpha, double 
     return MDBAS_NB_ERR_UNSUPPORTED;
   }
   const size_t smemF = sizeof(double) * 2 * (size_t)(M3 + 1) * fThreads;
-  MDB_TRY(c.t12.ensure(sizeof(double) * 2 * (size_t)(M1 + M2 + 2) * n));
   MDB_TRY(c.S.ensure(sizeof(double2) * (size_t)(K > 0 ? K : 1)));
   MDB_TRY(c.sums.ensure(sizeof(double) * 8));
+  const double rVol = kTwoPi / box->vol;
+  const double fact1 = 2.0 * rVol * chargeConst;
+  const double fact0 = 2.0 * fact1;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int parts = 0;
   if (K == 0) MDB_CUDA(cudaMemsetAsync(c.sums.p, 0, sizeof(double) * 8, s));
   if (K > 0) {
+    MDB_TRY(c.tab.ensure(sizeof(double) * 2 * (size_t)(M1 + M2 + M3 + 3) * n));
+    double *tab = c.tab.as<double>();
+    MDB_LAUNCH(k_ewald_tables, dim3(grid_for(n, 128), 3), 128, 0, s, n, b, M1, M2, M3, x, y, z,
+               tab);
     const int kBlocks = (K + kSfThreads - 1) / kSfThreads;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int P = (4 * sms + kBlocks - 1) / kBlocks;
     P = P < 1 ? 1 : P > 32 ? 32 : P;
     if (P > n) P = n;
@@ -394,22 +434,29 @@ int ewald_launch_impl(EwaldWork &c, int n, const PBC *box, double alpha, double 
     MDB_TRY(c.part.ensure(sizeof(double) * 2 * (size_t)P * K));
     const int kdBlocks = (K + 255) / 256;
     MDB_TRY(c.bpart.ensure(sizeof(double) * 7 * (size_t)kdBlocks));
-    MDB_LAUNCH(k_ewald_sf, dim3(kBlocks, P), kSfThreads, smemSf, s, n, K, perPart, tile, b, M1,
-               M2, M3, kl.km.as<int4>(), x, y, z, q, c.part.as<double>());
+    if (!c.done.p) {
+      MDB_TRY(c.done.ensure(sizeof(unsigned)));
+      MDB_CUDA(cudaMemsetAsync(c.done.p, 0, sizeof(unsigned), s));
+    }
+    MDB_LAUNCH(k_ewald_sf, dim3(kBlocks, P), kSfThreads, smemSf, s, n, K, perPart, tile, M1, M2,
+               M3, kl.km.as<int4>(), tab, q, c.part.as<double>());
     MDB_LAUNCH(k_ewald_kdata, kdBlocks, 256, 0, s, K, P, c.part.as<double>(),
                kl.kv.as<double4>(), kl.vam.as<double>(), c.S.as<double2>(),
-               c.bpart.as<double>());
-    MDB_LAUNCH(k_ewald_finish, 1, 256, 0, s, kdBlocks, c.bpart.as<double>(),
-               c.sums.as<double>());
+               c.bpart.as<double>(), c.done.as<unsigned>(), c.sums.as<double>());
+    // parts of the k list until there are four blocks for every SM
+    const int blocks = grid_for(n, fThreads);
+    parts = 1;
+    while (parts < kEwParts && (long long)blocks * parts < 4 * sms) parts *= 2;
+    MDB_TRY(c.pf.ensure(sizeof(double) * 3 * (size_t)parts * n));
+    MDB_CUDA(cudaFuncSetAttribute(k_ewald_forces, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smemF));
+    MDB_LAUNCH(k_ewald_forces, dim3(blocks, parts), fThreads, smemF, s, n, M1, M2, M3,
+               kEwParts / parts, kl.rowPart.as<int>(), kl.rows.as<int4>(), kl.rowK.as<int>(),
+               kl.rowBase.as<double4>(), kTwoPi * box->w1, kTwoPi * box->w2, kTwoPi * box->w3,
+               c.S.as<double2>(), tab, q, c.pf.as<double>());
   }
-  const double rVol = kTwoPi / box->vol;
-  const double fact1 = 2.0 * rVol * chargeConst;
-  const double fact0 = 2.0 * fact1;
-  MDB_CUDA(cudaFuncSetAttribute(k_ewald_forces, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smemF));
-  MDB_LAUNCH(k_ewald_forces, grid_for(n, fThreads), fThreads, smemF, s, n, b, M1, M2, M3,
-             kl.nRows, kl.rows.as<int4>(), kl.rowK.as<int>(), kl.kv.as<double4>(),
-             c.S.as<double2>(), x, y, z, q, c.t12.as<double>(), fact0, scaleInput, fx, fy, fz);
+  MDB_LAUNCH(k_ewald_add, dim3(grid_for(n, 256), 3), 256, 0, s, n, parts, c.pf.as<double>(), fact0,
+             scaleInput, fx, fy, fz);
   c.fact1 = fact1;
   return MDBAS_NB_OK;
 }

@@ -14,13 +14,13 @@ struct EwaldKList {
   double key[12] = {};
   int M1 = 0, M2 = 0, M3 = 0;
   int K = 0, nRows = 0;
-  DBuf km, kv, vam, rows, rowK;
+  DBuf km, kv, vam, rows, rowK, rowBase, rowPart;
 };
 
 struct EwaldWork {
   EwaldKList kl;
   int device = -1;
-  DBuf part, S, bpart, sums, t12, xyzq, f;
+  DBuf part, S, bpart, sums, tab, pf, done, xyzq, f;
   double fact1 = 0.;  // 2 (2 pi / V) C of the last launch
 };
 
