@@ -24,22 +24,27 @@ struct EwaldWork {
   double fact1 = 0.;  // 2 (2 pi / V) C of the last launch
 };
 
+constexpr int kSpmeEnergy = 6;  // SpmeWork::sums: 0-5 stress, 6 energy, 7-9 force sums
 struct SpmeWork {
   int device = -1;
   int m1 = 0, m2 = 0, m3 = 0, nbsp = 0, n = 0;
-  cufftHandle plan = 0;
-  bool planValid = false;
+  cufftHandle plan = 0, planBack = 0;  // D2Z, Z2D
+  bool planValid = false, planBackValid = false;
   DBuf qsp, ft, bmod, spl, cell, fr, sums, xyzq, fout;
   // deterministic spreading: atoms binned by the 8^3 grid tile of their
   // base cell, each tile's atoms in ascending index order
-  DBuf tileOf, tileCount, tileStart, tileFill, tileList, tileSorted, scanTmp;
+  DBuf tileOf, tileCount, tileStart, tileFill, tileList, tileSorted;
   DBuf halo;         // per tile: the (8 + p - 1)^3 halo box of its atoms' stencils
   int haloSmem = 0;  // dynamic shared memory the halo kernel is allowed
   DBuf part;         // per-block partial sums (fixed-order reductions)
+  DBuf done;         // their finished-blocks counter
   double f1 = 0.;  // (2 pi / V) C of the last launch
-  ~SpmeWork() {
+  void drop_plans() {
     if (planValid) cufftDestroy(plan);
+    if (planBackValid) cufftDestroy(planBack);
+    planValid = planBackValid = false;
   }
+  ~SpmeWork() { drop_plans(); }
 };
 
 // Explicit Ewald reciprocal forces added to fx/fy/fz (device arrays; with
@@ -52,7 +57,7 @@ int ewald_launch(EwaldWork &c, int n, const PBC *box, double alpha, double charg
                  const double *q, double *fx, double *fy, double *fz, int scaleInput,
                  cudaStream_t s);
 // SPME reciprocal forces minus their mean added to fx/fy/fz (device arrays);
-// c.sums[9] = the grid energy sum, c.sums[0..5] stress sums.  Capturable
+// c.sums[kSpmeEnergy] = the grid energy sum, c.sums[0..5] stress sums.  Capturable
 // once the plan and buffers exist for these arguments.
 int spme_launch(SpmeWork &c, int n, const PBC *box, double alpha, double chargeConst, int m1,
                 int m2, int m3, int nbsp, const double *x, const double *y, const double *z,

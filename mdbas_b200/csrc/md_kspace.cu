@@ -39,7 +39,7 @@ int kspace_launch(mdbas_nb_engine *e, double *f, cudaStream_t s) {
   MDB_TRY(spme_launch(*e->kSpme, n, &e->hostBox, e->cfg.alpha, e->cfg.chargeConst,
                       e->kspaceM[0], e->kspaceM[1], e->kspaceM[2], e->kspaceOrder, x, y, z, q, f,
                       fy, fz, s));
-  return kspace_fix_launch(e->kSpme->sums.as<double>() + 9, e->kSpme->f1, kspace_enn(e),
+  return kspace_fix_launch(e->kSpme->sums.as<double>() + kSpmeEnergy, e->kSpme->f1, kspace_enn(e),
                            e->kspaceFix.as<long long>(), s);
 }
 
@@ -136,7 +136,7 @@ int mdbas_nb_engine_kspace(mdbas_nb_engine *e, double *fx, double *fy, double *f
     st5 = fct * (sums[6] + erec) + enn;
   } else {
     fct = e->kSpme->f1;
-    erec = sums[9];
+    erec = sums[kSpmeEnergy];
     st0 = fct * (sums[0] + erec) + enn;
     st3 = fct * (sums[3] + erec) + enn;
     st5 = fct * (sums[5] + erec) + enn;
