@@ -179,8 +179,29 @@ __device__ __forceinline__ PairTerms pair_ewald_fast(const PairParams &p, const 
 constexpr double kFastR2Min = 1e-6;
 constexpr int kPairBlocks = 6;    // blocks per SM
 
-// acc[0..4]: elec, vdw, virelec, virvdw, in-cut-off pairs; acc[7]: the work
-// counter.
+// The sum of every block's v into acc[c], without the rounding of one FP64
+// addition after the other (a thousand blocks' would show in differences of
+// energies): multiples of 2^-10 and what is left of v, in multiples of 2^-60,
+// are added as integers, and the last block puts them together.  A sum too
+// large for that is added as it is.
+__device__ __forceinline__ void exact_add(double *acc, int c, double v) {
+  if (!(fabs(v) < 1e12)) {
+    atomicAdd(acc + c, v);
+    return;
+  }
+  const long long h = __double2ll_rn(v * 1024.);
+  const double rest = v - (double)h * (1. / 1024.);
+  red_add(reinterpret_cast<long long *>(acc + 8 + 2 * c), h);
+  red_add(reinterpret_cast<long long *>(acc + 9 + 2 * c),
+          __double2ll_rn(rest * 1152921504606846976.));
+}
+__device__ __forceinline__ void exact_finish(double *acc, int c) {
+  const long long h = __ldcg(reinterpret_cast<long long *>(acc + 8 + 2 * c));
+  const long long l = __ldcg(reinterpret_cast<long long *>(acc + 9 + 2 * c));
+  atomicAdd(acc + c, (double)h * (1. / 1024.) + (double)l * (1. / 1152921504606846976.));
+}
+
+// acc: see pair_fp64.cuh.
 //
 // The row walk of pair_rows.cuh; warps keep their energy sums in registers
 // over all their atoms.  Bound by latency and the LSU (gathers and scattered
@@ -262,7 +283,17 @@ k_pairs_fp64(int n, DevBox b, PairParams p, HalfList hl, const double *__restric
   if (threadIdx.x < 5) {
     double v = 0.;
     for (int c = 0; c < kRowWarps; ++c) v += red[threadIdx.x][c];
-    atomicAdd(acc + threadIdx.x, v);
+    exact_add(acc, threadIdx.x, v);
+    __threadfence();
+  }
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicAdd(reinterpret_cast<unsigned *>(acc + 7) + 1, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last && threadIdx.x < 5) {
+    __threadfence();
+    exact_finish(acc, threadIdx.x);
   }
 }
 

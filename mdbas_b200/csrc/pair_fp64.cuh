@@ -6,11 +6,12 @@
 namespace mdbas {
 
 // Accumulator layout (FP64, device): 0 elec, 1 vdw, 2 virelec, 3 virvdw,
-// 4 in-cut-off pairs, 5 eCorr, 6 virCorr, 7 work counter of the pair kernel.
-constexpr int kFp64AccCount = 8;
+// 4 in-cut-off pairs, 5 eCorr, 6 virCorr; the pair kernel's own: 7 its work and
+// finished-blocks counters, 8.. the sums 0-4 in two fixed-point parts.
+constexpr int kFp64AccCount = 24;
 
 // Pair loop over the half list; forces are added to fx/fy/fz, sums to acc
-// (acc[7] zero on entry).
+// (all zero on entry).
 int pairs_fp64(int ewald, int n, const DevBox &b, const PairParams &p, const int *order,
                const int *neighPair, const long long *off, const int *list, const double *x,
                const double *y, const double *z, const double *q, const double *eps,
