@@ -15,6 +15,7 @@
 // the adjoint is the gradient harness's reference-quality path.
 #include "common.cuh"
 #include "engine.cuh"
+#include "host_copy.cuh"
 #include "pair_rows.cuh"
 #include "real64.cuh"
 
@@ -290,13 +291,16 @@ extern "C" int mdbas_nb_engine_adjoint(mdbas_nb_engine *e, const double *vx, con
   double *buf = e->adjBuf.as<double>();
   double *dv = buf, *outs = buf + 3 * (size_t)n;
   MDB_CUDA(cudaMemsetAsync(outs, 0, sizeof(double) * (9 * (size_t)n + 1), s));
-  const cudaMemcpyKind in = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  const cudaMemcpyKind outk = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   const size_t bytes = sizeof(double) * (size_t)n;
-  if (hvp) {
-    MDB_CUDA(cudaMemcpyAsync(dv, vx, bytes, in, s));
-    MDB_CUDA(cudaMemcpyAsync(dv + n, vy, bytes, in, s));
-    MDB_CUDA(cudaMemcpyAsync(dv + 2 * (size_t)n, vz, bytes, in, s));
+  if (hvp && device_ptrs) {
+    const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
+    MDB_CUDA(cudaMemcpyAsync(dv, vx, bytes, k, s));
+    MDB_CUDA(cudaMemcpyAsync(dv + n, vy, bytes, k, s));
+    MDB_CUDA(cudaMemcpyAsync(dv + 2 * (size_t)n, vz, bytes, k, s));
+  } else if (hvp) {
+    const CopySpan3 in(const_cast<double *>(vx), const_cast<double *>(vy),
+                       const_cast<double *>(vz), dv, n);
+    MDB_TRY(copy_in(in.s, 3, s));
   }
   AdjOut o;
   double *const ptrs[9] = {outs, outs + n, outs + 2 * (size_t)n, outs + 3 * (size_t)n,
@@ -319,8 +323,14 @@ extern "C" int mdbas_nb_engine_adjoint(mdbas_nb_engine *e, const double *vx, con
              e->exclStart.as<int>(), e->exclFlat.as<int>(), e->x.as<double>(),
              e->y.as<double>(), e->z.as<double>(), e->q.as<double>(), dvx, dvy, dvz, o);
   double *dst[9] = {gq, geps, gsig, hx, hy, hz, pq, peps, psig};
-  for (int k = 0; k < (hvp ? 9 : 3); ++k)
-    MDB_CUDA(cudaMemcpyAsync(dst[k], ptrs[k], bytes, outk, s));
+  const int outputs = hvp ? 9 : 3;
+  if (!device_ptrs) {
+    CopySpan out[9];
+    for (int k = 0; k < outputs; ++k) out[k] = CopySpan(dst[k], ptrs[k], bytes, false, k > 0);
+    return copy_out(out, outputs, s);
+  }
+  for (int k = 0; k < outputs; ++k)
+    MDB_CUDA(cudaMemcpyAsync(dst[k], ptrs[k], bytes, cudaMemcpyDeviceToDevice, s));
   MDB_CUDA(cudaStreamSynchronize(s));
   return MDBAS_NB_OK;
 }

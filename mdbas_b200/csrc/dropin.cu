@@ -29,6 +29,7 @@
 
 #include "cluster.cuh"
 #include "engine.cuh"
+#include "host_copy.cuh"
 #include "list_ref.cuh"
 #include "pair_fp32.cuh"
 #include "pair_fp64.cuh"
@@ -128,10 +129,6 @@ struct Ctx {
   DevBox clBox{};
   int elecType = FULL, vdwType = VSWITCH;
   bool ptrsSet = false;
-  // page-locked staging for the positions going up and the forces coming
-  // down (the caller's arrays are pageable), grown on demand
-  double *pinIn = nullptr, *pinOut = nullptr;
-  size_t pinInCap = 0, pinOutCap = 0;
 };
 
 Ctx g;
@@ -143,6 +140,7 @@ int ctx_init() {
   ST_TRY(engine_check_device(g.device));
   MDB_CUDA(cudaSetDevice(g.device));
   MDB_CUDA(cudaStreamCreateWithFlags(&g.s, cudaStreamNonBlocking));
+  host_copy_enter();  // the context lives as long as the process
   g.ready = true;
   return MDBAS_NB_OK;
 }
@@ -152,34 +150,15 @@ bool resident_enabled() {
   return !(v && v[0] == '0');
 }
 
-// Page-locked host buffer of at least `count` doubles.  Every call that uses
-// one ends with a stream synchronisation, so a buffer is never refilled while
-// a copy from or into it is in flight.
-int pinned(double *&buf, size_t &cap, size_t count) {
-  if (cap >= count && buf) return MDBAS_NB_OK;
-  if (buf) cudaFreeHost(buf);
-  buf = nullptr;
-  cap = 0;
-  MDB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&buf), sizeof(double) * count,
-                         cudaHostAllocDefault));
-  cap = count;
-  return MDBAS_NB_OK;
-}
-
 int upload_positions(int n, const double *x, const double *y, const double *z) {
   ST_TRY(g.x.ensure(sizeof(double) * n));
   ST_TRY(g.y.ensure(sizeof(double) * n));
   ST_TRY(g.z.ensure(sizeof(double) * n));
-  ST_TRY(pinned(g.pinIn, g.pinInCap, 3 * (size_t)n));
-  double *h = g.pinIn;
-  memcpy(h, x, sizeof(double) * n);
-  memcpy(h + n, y, sizeof(double) * n);
-  memcpy(h + 2 * (size_t)n, z, sizeof(double) * n);
-  MDB_CUDA(cudaMemcpyAsync(g.x.p, h, sizeof(double) * n, cudaMemcpyHostToDevice, g.s));
-  MDB_CUDA(cudaMemcpyAsync(g.y.p, h + n, sizeof(double) * n, cudaMemcpyHostToDevice, g.s));
-  MDB_CUDA(cudaMemcpyAsync(g.z.p, h + 2 * (size_t)n, sizeof(double) * n,
-                           cudaMemcpyHostToDevice, g.s));
-  return MDBAS_NB_OK;
+  const size_t bytes = sizeof(double) * (size_t)n;
+  const CopySpan in[3] = {{const_cast<double *>(x), g.x.p, bytes},
+                          {const_cast<double *>(y), g.y.p, bytes},
+                          {const_cast<double *>(z), g.z.p, bytes}};
+  return copy_in(in, 3, g.s);
 }
 
 int upload_vec(DBuf &d, std::vector<double> &cache, const double *h, int n) {
@@ -282,15 +261,25 @@ void print_grow(int from, int to) {
 }
 
 // FNV-1a style hash of neighPair and of every 61st list entry plus the last
-// ones: a guard against arrays refilled since the library's build.
+// ones: a guard against arrays refilled since the library's build.  Eight
+// hashes side by side, one multiplication after the other in each.
 unsigned long long list_checksum(int n, const int *neighList, const int *neighPair,
                                  long long total) {
-  unsigned long long h = 1469598103934665603ull;
-  auto mix = [&h](unsigned v) { h = (h ^ v) * 1099511628211ull; };
-  for (int i = 0; i < n; ++i) mix((unsigned)neighPair[i]);
-  for (long long k = 0; k < total; k += 61) mix((unsigned)neighList[k]);
-  for (long long k = total > 64 ? total - 64 : 0; k < total; ++k) mix((unsigned)neighList[k]);
-  return h;
+  unsigned long long h[8];
+  for (int k = 0; k < 8; ++k) h[k] = 1469598103934665603ull + k;
+  const auto mix = [](unsigned long long &v, unsigned x) { v = (v ^ x) * 1099511628211ull; };
+  const auto range = [&](const int *p, long long first, long long last, long long step) {
+    long long k = first;
+    for (; k + 7 * step < last; k += 8 * step)
+      for (int l = 0; l < 8; ++l) mix(h[l], (unsigned)p[k + l * step]);
+    for (int l = 0; k < last; k += step, ++l) mix(h[l], (unsigned)p[k]);
+  };
+  range(neighPair, 0, n, 1);
+  range(neighList, 0, total, 61);
+  range(neighList, total > 64 ? total - 64 : 0, total, 1);
+  unsigned long long s = 1469598103934665603ull;
+  for (int k = 0; k < 8; ++k) s = (s ^ h[k]) * 1099511628211ull;
+  return s;
 }
 
 // Build MDBas's list on the device and hand it to the caller's arrays.
@@ -355,15 +344,10 @@ int list_common(int linkCells, int first, PARAM *param, PBC *box, NEIGH *neigh, 
     pairArr = neighPairArr;
     orderArr = neighOrderArr;
   }
-  if (total > 0)
-    MDB_CUDA(cudaMemcpyAsync(*neighList, g.ref.list.p, sizeof(int) * total,
-                             cudaMemcpyDeviceToHost, g.s));
-  MDB_CUDA(cudaMemcpyAsync(pairArr, g.ref.neighPair.p, sizeof(int) * n, cudaMemcpyDeviceToHost,
-                           g.s));
-  if (orderArr)
-    MDB_CUDA(cudaMemcpyAsync(orderArr, g.ref.order.p, sizeof(int) * n, cudaMemcpyDeviceToHost,
-                             g.s));
-  MDB_CUDA(cudaStreamSynchronize(g.s));
+  const CopySpan out[3] = {{*neighList, g.ref.list.p, sizeof(int) * (size_t)total},
+                           {pairArr, g.ref.neighPair.p, sizeof(int) * (size_t)n},
+                           {orderArr, g.ref.order.p, sizeof(int) * (size_t)n}};
+  ST_TRY(copy_out(out, orderArr ? 3 : 2, g.s));
   g.resList = *neighList;
   g.resPair = pairArr;
   g.resOrder = orderArr;
@@ -387,13 +371,11 @@ int ensure_list_on_device(int n, const int *neighList, const int *neighPair,
   ST_TRY(g.ref.list.ensure(sizeof(int) * (size_t)std::max<long long>(1, total)));
   ST_TRY(g.ref.neighPair.ensure(sizeof(int) * n));
   ST_TRY(g.ref.order.ensure(sizeof(int) * n));
-  if (total > 0)
-    MDB_CUDA(cudaMemcpyAsync(g.ref.list.p, neighList, sizeof(int) * total, cudaMemcpyHostToDevice,
-                             g.s));
-  MDB_CUDA(cudaMemcpyAsync(g.ref.neighPair.p, neighPair, sizeof(int) * n, cudaMemcpyHostToDevice,
-                           g.s));
-  MDB_CUDA(cudaMemcpyAsync(g.ref.order.p, neighOrder, sizeof(int) * n, cudaMemcpyHostToDevice,
-                           g.s));
+  const CopySpan in[3] = {
+      {const_cast<int *>(neighList), g.ref.list.p, sizeof(int) * (size_t)total},
+      {const_cast<int *>(neighPair), g.ref.neighPair.p, sizeof(int) * (size_t)n},
+      {const_cast<int *>(neighOrder), g.ref.order.p, sizeof(int) * (size_t)n}};
+  ST_TRY(copy_in(in, 3, g.s));
   ST_TRY(ref_list_offsets(g.ref, n, g.s));
   g.resList = neighList;
   g.resPair = neighPair;
@@ -404,19 +386,13 @@ int ensure_list_on_device(int n, const int *neighList, const int *neighPair,
   return MDBAS_NB_OK;
 }
 
-// Download device forces and add them into the caller's arrays.
-int add_forces(int n, const double *dsrc, double *fx, double *fy, double *fz) {
-  ST_TRY(pinned(g.pinOut, g.pinOutCap, 3 * (size_t)n));
-  MDB_CUDA(cudaMemcpyAsync(g.pinOut, dsrc, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost,
-                           g.s));
-  MDB_CUDA(cudaStreamSynchronize(g.s));
-  const double *h = g.pinOut;
-  for (int i = 0; i < n; ++i) {
-    fx[i] += h[i];
-    fy[i] += h[n + i];
-    fz[i] += h[2 * n + i];
-  }
-  return MDBAS_NB_OK;
+// Download device forces and add them into the caller's arrays; `sums` (bytes
+// from dsums) come with them.
+int add_forces(int n, const double *dsrc, double *fx, double *fy, double *fz, void *sums = nullptr,
+               const void *dsums = nullptr, size_t sumBytes = 0) {
+  const CopySpan3 f3(fx, fy, fz, const_cast<double *>(dsrc), n, true);
+  const CopySpan out[4] = {f3.s[0], f3.s[1], f3.s[2], {sums, const_cast<void *>(dsums), sumBytes}};
+  return copy_out(out, sums ? 4 : 3, g.s);
 }
 
 // What the cluster list needs for these positions: a rebuild (max
@@ -480,8 +456,7 @@ int real_space(int mode, int listRule, int n, const PARAM *param, double alpha, 
                      g.y.as<double>(), g.z.as<double>(), g.q.as<double>(), fxd, fyd, fzd,
                      g.acc64.as<double>(), g.s));
     double a[kFp64AccCount];
-    MDB_CUDA(cudaMemcpyAsync(a, g.acc64.p, sizeof(a), cudaMemcpyDeviceToHost, g.s));
-    ST_TRY(add_forces(n, g.f3.as<double>(), fx, fy, fz));
+    ST_TRY(add_forces(n, g.f3.as<double>(), fx, fy, fz, a, g.acc64.p, sizeof(a)));
     e[0] = a[0];
     e[1] = a[5];
     e[2] = a[1];
@@ -522,8 +497,7 @@ int real_space(int mode, int listRule, int n, const PARAM *param, double alpha, 
   double *fxd = g.f3.as<double>();
   ST_TRY(forces_out_launch(w, n, 0, fxd, fxd + n, fxd + 2 * (size_t)n, g.s));
   long long a[ACC_COUNT];
-  MDB_CUDA(cudaMemcpyAsync(a, w.acc.p, sizeof(a), cudaMemcpyDeviceToHost, g.s));
-  ST_TRY(add_forces(n, fxd, fx, fy, fz));
+  ST_TRY(add_forces(n, fxd, fx, fy, fz, a, w.acc.p, sizeof(a)));
   if (a[ACC_FLAGS] & FLAG_OVERFLOW) return MDBAS_NB_ERR_OVERFLOW;
   const double inv = 1.0 / kEnergyScale;
   e[0] = (double)a[ACC_E_DIR] * inv;
@@ -870,8 +844,7 @@ void nonbond_energy(PARAM *param, ENERGY *ener, PBC *box, const double x[], cons
                       g.sig.as<double>(), fxd, fxd + n, fxd + 2 * (size_t)n, g.acc64.as<double>(),
                       g.s));
     double a[kFp64AccCount];
-    MDB_CUDA(cudaMemcpyAsync(a, g.acc64.p, sizeof(a), cudaMemcpyDeviceToHost, g.s));
-    ST_TRY(add_forces(n, fxd, fx, fy, fz));
+    ST_TRY(add_forces(n, fxd, fx, fy, fz, a, g.acc64.p, sizeof(a)));
     ener->elec += a[0];
     ener->vdw += a[1];
     ener->virelec += a[2];

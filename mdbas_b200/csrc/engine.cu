@@ -12,6 +12,7 @@
 
 #include "cluster.cuh"
 #include "engine.cuh"
+#include "host_copy.cuh"
 #include "list_ref.cuh"
 #include "pair_fp32.cuh"
 #include "pair_fp64.cuh"
@@ -237,6 +238,8 @@ int mdbas_nb_engine_create(mdbas_nb_engine **out, const mdbas_nb_engine_config *
     return MDBAS_NB_ERR_CUDA;
   }
   e->ownStream = true;
+  host_copy_enter();
+  e->hostCopy = true;
   cudaEventCreate(&e->ev0);
   cudaEventCreate(&e->ev1);
   if (upload_boxes(e) != MDBAS_NB_OK) {
@@ -300,6 +303,7 @@ int mdbas_nb_engine_destroy(mdbas_nb_engine *e) {
     cudaEventDestroy(e->evJoin);
   }
   if (e->ownStream) cudaStreamDestroy(e->stream);
+  if (e->hostCopy) host_copy_leave();
   delete e;
   return MDBAS_NB_OK;
 }
@@ -351,23 +355,22 @@ int mdbas_nb_engine_set_topology(mdbas_nb_engine *e, const double *q, const doub
   ENG_TRY(e, e->exclStart.ensure(sizeof(int) * (n + 1)));
   ENG_TRY(e, e->exclFlat.ensure(sizeof(int) * (nex > 0 ? nex : 1)));
   cudaStream_t s = e->stream;
-  MDB_CUDA(cudaMemcpyAsync(e->q.p, q, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(e->eps.p, eps, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(e->sig.p, sig, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(e->exclStart.p, start.data(), sizeof(int) * (n + 1),
-                           cudaMemcpyHostToDevice, s));
-  if (nex > 0)
-    MDB_CUDA(cudaMemcpyAsync(e->exclFlat.p, exclFlat, sizeof(int) * nex, cudaMemcpyHostToDevice,
-                             s));
   // the cluster search reads each excluded pair from both atoms' rows
   cluster_symmetric_excl(n, start.data(), exclFlat, e->hExclStartSym, e->hExclFlatSym);
   ENG_TRY(e, e->exclStartSym.ensure(sizeof(int) * (n + 1)));
   ENG_TRY(e, e->exclFlatSym.ensure(sizeof(int) * std::max<size_t>(1, e->hExclFlatSym.size())));
-  MDB_CUDA(cudaMemcpyAsync(e->exclStartSym.p, e->hExclStartSym.data(), sizeof(int) * (n + 1),
-                           cudaMemcpyHostToDevice, s));
-  if (!e->hExclFlatSym.empty())
-    MDB_CUDA(cudaMemcpyAsync(e->exclFlatSym.p, e->hExclFlatSym.data(),
-                             sizeof(int) * e->hExclFlatSym.size(), cudaMemcpyHostToDevice, s));
+  {
+    const size_t bytes = sizeof(double) * (size_t)n, rows = sizeof(int) * (size_t)(n + 1);
+    const CopySpan in[7] = {
+        {const_cast<double *>(q), e->q.p, bytes},
+        {const_cast<double *>(eps), e->eps.p, bytes},
+        {const_cast<double *>(sig), e->sig.p, bytes},
+        {start.data(), e->exclStart.p, rows},
+        {const_cast<int *>(exclFlat), e->exclFlat.p, sizeof(int) * (size_t)nex},
+        {e->hExclStartSym.data(), e->exclStartSym.p, rows},
+        {e->hExclFlatSym.data(), e->exclFlatSym.p, sizeof(int) * e->hExclFlatSym.size()}};
+    ENG_TRY(e, copy_in(in, 7, s));
+  }
   e->hasFrozen = false;
   if (frozen) {
     bool any = false;
@@ -407,10 +410,18 @@ int mdbas_nb_engine_set_positions(mdbas_nb_engine *e, const double *x, const dou
   ENG_TRY(e, e->x.ensure(sizeof(double) * n));
   ENG_TRY(e, e->y.ensure(sizeof(double) * n));
   ENG_TRY(e, e->z.ensure(sizeof(double) * n));
-  const cudaMemcpyKind k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  MDB_CUDA(cudaMemcpyAsync(e->x.p, x, sizeof(double) * n, k, e->stream));
-  MDB_CUDA(cudaMemcpyAsync(e->y.p, y, sizeof(double) * n, k, e->stream));
-  MDB_CUDA(cudaMemcpyAsync(e->z.p, z, sizeof(double) * n, k, e->stream));
+  const size_t bytes = sizeof(double) * (size_t)n;
+  if (device_ptrs) {
+    const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
+    MDB_CUDA(cudaMemcpyAsync(e->x.p, x, bytes, k, e->stream));
+    MDB_CUDA(cudaMemcpyAsync(e->y.p, y, bytes, k, e->stream));
+    MDB_CUDA(cudaMemcpyAsync(e->z.p, z, bytes, k, e->stream));
+  } else {
+    const CopySpan in[3] = {{const_cast<double *>(x), e->x.p, bytes},
+                            {const_cast<double *>(y), e->y.p, bytes},
+                            {const_cast<double *>(z), e->z.p, bytes}};
+    ENG_TRY(e, copy_in(in, 3, e->stream));
+  }
   e->posSet = true;
   return MDBAS_NB_OK;
 }
@@ -555,25 +566,26 @@ int mdbas_nb_engine_get_forces(mdbas_nb_engine *e, double *fx, double *fy, doubl
       src = e->fout.as<double>();
       ENG_TRY(e, forces_out_launch(e->cl, n, 0, src, src + n, src + 2 * (size_t)n, s));
     }
-    const cudaMemcpyKind k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    MDB_CUDA(cudaMemcpyAsync(fx, src, sizeof(double) * n, k, s));
-    MDB_CUDA(cudaMemcpyAsync(fy, src + n, sizeof(double) * n, k, s));
-    MDB_CUDA(cudaMemcpyAsync(fz, src + 2 * (size_t)n, sizeof(double) * n, k, s));
-    if (device_ptrs) return MDBAS_NB_OK;
+    const size_t bytes = sizeof(double) * (size_t)n;
+    if (device_ptrs) {
+      const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
+      MDB_CUDA(cudaMemcpyAsync(fx, src, bytes, k, s));
+      MDB_CUDA(cudaMemcpyAsync(fy, src + n, bytes, k, s));
+      MDB_CUDA(cudaMemcpyAsync(fz, src + 2 * (size_t)n, bytes, k, s));
+      return MDBAS_NB_OK;
+    }
     // the energy words ride along with the forces: one wait for both, and the
     // fixed-point error bits checked here too
-    if (e->cfg.precision == 0)
-      MDB_CUDA(cudaMemcpyAsync(e->acc64Cache, e->acc64.p, sizeof(e->acc64Cache),
-                               cudaMemcpyDeviceToHost, s));
-    else
-      MDB_CUDA(cudaMemcpyAsync(e->accCache, e->cl.acc.p, sizeof(e->accCache),
-                               cudaMemcpyDeviceToHost, s));
     long long sticky = 0;
     const bool settle = settleAfter && pass == 0 && e->buildPending;
-    if (settle)
-      MDB_CUDA(cudaMemcpyAsync(&sticky, e->cl.sticky.p, sizeof(sticky), cudaMemcpyDeviceToHost,
-                               s));
-    MDB_CUDA(cudaStreamSynchronize(s));
+    const CopySpan3 f3(fx, fy, fz, src, n);
+    CopySpan out[5] = {f3.s[0], f3.s[1], f3.s[2]};
+    if (e->cfg.precision == 0)
+      out[3] = {e->acc64Cache, e->acc64.p, sizeof(e->acc64Cache)};
+    else
+      out[3] = {e->accCache, e->cl.acc.p, sizeof(e->accCache)};
+    out[4] = {&sticky, e->cl.sticky.p, sizeof(sticky)};
+    ENG_TRY(e, copy_out(out, settle ? 5 : 4, s));
     if (!settle) break;
     e->buildPending = false;
     if (!(sticky & (CL_OVERFLOW | CL_NONFINITE))) break;

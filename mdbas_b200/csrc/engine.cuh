@@ -24,6 +24,7 @@ struct mdbas_nb_engine {
   mdbas::PairParams pp{};
   cudaStream_t stream = nullptr;
   bool ownStream = false;
+  bool hostCopy = false;  // registered with the page-locked chunks (host_copy.cuh)
   // topology (caller's atom order)
   mdbas::DBuf q, eps, sig, frozen, exclStart, exclFlat;
   // the exclusion rows made symmetric (each excluded pair in both atoms'

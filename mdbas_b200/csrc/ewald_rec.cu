@@ -26,6 +26,7 @@
 
 #include <vector>
 
+#include "host_copy.cuh"
 #include "kspace.cuh"
 
 namespace mdbas {
@@ -461,20 +462,10 @@ int ewald_launch_impl(EwaldWork &c, int n, const PBC *box, double alpha, double 
   return MDBAS_NB_OK;
 }
 
-// Device arrays; out[0] = energy (reciprocal + self + non-neutral), out[1] =
-// virial, out[2..7] = stress.
-int ewald_run(int n, const PBC *box, double alpha, double chargeConst, int M1, int M2, int M3,
-              const double *x, const double *y, const double *z, const double *q, double systq,
-              double sumq2, double *fx, double *fy, double *fz, int scaleInput, double out[8],
-              cudaStream_t s) {
-  EwaldWork &c = ewald_ctx();
-  MDB_TRY(ewald_launch_impl(c, n, box, alpha, chargeConst, M1, M2, M3, x, y, z, q, fx, fy, fz,
-                            scaleInput, s));
-  double h[7];
-  MDB_CUDA(cudaMemcpyAsync(h, c.sums.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-  MDB_CUDA(cudaStreamSynchronize(s));
-  const double fact1 = c.fact1;
-  // src/ewald.c:323-352
+// out[0] = energy (reciprocal + self + non-neutral), out[1] = virial,
+// out[2..7] = stress, from the device sums h (src/ewald.c:323-352).
+void ewald_results(double fact1, const PBC *box, double alpha, double chargeConst, double systq,
+                   double sumq2, const double *h, double out[8]) {
   const double eself = -chargeConst * alpha * sumq2 / kSqrtPi;
   const double enn = -(0.5 * kPi * chargeConst) * ((systq / alpha) * (systq / alpha) / box->vol);
   const double etmp = h[0];
@@ -488,6 +479,20 @@ int ewald_run(int n, const PBC *box, double alpha, double chargeConst, int M1, i
   out[0] = fact1 * etmp + eself + enn;
   out[1] = -(st[0] + st[3] + st[5]);
   for (int k = 0; k < 6; ++k) out[2 + k] = st[k];
+}
+
+// Device arrays.
+int ewald_run(int n, const PBC *box, double alpha, double chargeConst, int M1, int M2, int M3,
+              const double *x, const double *y, const double *z, const double *q, double systq,
+              double sumq2, double *fx, double *fy, double *fz, int scaleInput, double out[8],
+              cudaStream_t s) {
+  EwaldWork &c = ewald_ctx();
+  MDB_TRY(ewald_launch_impl(c, n, box, alpha, chargeConst, M1, M2, M3, x, y, z, q, fx, fy, fz,
+                            scaleInput, s));
+  double h[7];
+  MDB_CUDA(cudaMemcpyAsync(h, c.sums.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+  MDB_CUDA(cudaStreamSynchronize(s));
+  ewald_results(c.fact1, box, alpha, chargeConst, systq, sumq2, h, out);
   return MDBAS_NB_OK;
 }
 
@@ -498,29 +503,29 @@ int ewald_host(int n, const PBC *box, double alpha, double chargeConst, int M1, 
                const double *x, const double *y, const double *z, const double *q, double *fx,
                double *fy, double *fz, int scaleInput, double out[8]) {
   EwaldWork &c = ewald_ctx();
-  double systq = 0., sumq2 = 0.;
-  for (int i = 0; i < n; ++i) {  // src/ewald.c:166-172
-    systq += q[i];
-    sumq2 += q[i] * q[i];
-  }
+  standalone_copies();
+  double systq, sumq2;
+  charge_sums(n, q, &systq, &sumq2);  // src/ewald.c:166-172
   cudaStream_t s = nullptr;
   MDB_TRY(c.xyzq.ensure(sizeof(double) * 4 * (size_t)n));
   MDB_TRY(c.f.ensure(sizeof(double) * 3 * (size_t)n));
   double *d = c.xyzq.as<double>(), *f = c.f.as<double>();
   const size_t bytes = sizeof(double) * (size_t)n;
-  MDB_CUDA(cudaMemcpyAsync(d, x, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(d + n, y, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(d + 2 * (size_t)n, z, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(d + 3 * (size_t)n, q, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(f, fx, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(f + n, fy, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(f + 2 * (size_t)n, fz, bytes, cudaMemcpyHostToDevice, s));
-  MDB_TRY(ewald_run(n, box, alpha, chargeConst, M1, M2, M3, d, d + n, d + 2 * (size_t)n,
-                    d + 3 * (size_t)n, systq, sumq2, f, f + n, f + 2 * (size_t)n, scaleInput,
-                    out, s));
-  MDB_CUDA(cudaMemcpy(fx, f, bytes, cudaMemcpyDeviceToHost));
-  MDB_CUDA(cudaMemcpy(fy, f + n, bytes, cudaMemcpyDeviceToHost));
-  MDB_CUDA(cudaMemcpy(fz, f + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost));
+  const CopySpan3 f3(fx, fy, fz, f, n);
+  const CopySpan in[7] = {
+      {const_cast<double *>(x), d, bytes},
+      {const_cast<double *>(y), d + n, bytes, false, true},
+      {const_cast<double *>(z), d + 2 * (size_t)n, bytes, false, true},
+      {const_cast<double *>(q), d + 3 * (size_t)n, bytes, false, true},
+      f3.s[0], f3.s[1], f3.s[2]};
+  MDB_TRY(copy_in(in, 7, s));
+  MDB_TRY(ewald_launch_impl(c, n, box, alpha, chargeConst, M1, M2, M3, d, d + n,
+                            d + 2 * (size_t)n, d + 3 * (size_t)n, f, f + n, f + 2 * (size_t)n,
+                            scaleInput, s));
+  double h[7];
+  const CopySpan o[4] = {f3.s[0], f3.s[1], f3.s[2], {h, c.sums.p, sizeof(h)}};
+  MDB_TRY(copy_out(o, 4, s));
+  ewald_results(c.fact1, box, alpha, chargeConst, systq, sumq2, h, out);
   return MDBAS_NB_OK;
 }
 
@@ -537,6 +542,31 @@ int ewald_launch(EwaldWork &c, int n, const PBC *box, double alpha, double charg
                  cudaStream_t s) {
   return ewald_launch_impl(c, n, box, alpha, chargeConst, M1, M2, M3, x, y, z, q, fx, fy, fz,
                            scaleInput, s);
+}
+
+void charge_sums(int n, const double *q, double *systq, double *sumq2) {
+  // eight sums side by side: one chain would take four cycles an atom
+  double a[8] = {}, b[8] = {};
+  int i = 0;
+  for (; i + 8 <= n; i += 8)
+    for (int k = 0; k < 8; ++k) {
+      a[k] += q[i + k];
+      b[k] += q[i + k] * q[i + k];
+    }
+  for (int k = 0; i < n; ++i, ++k) {
+    a[k] += q[i];
+    b[k] += q[i] * q[i];
+  }
+  *systq = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+  *sumq2 = ((b[0] + b[1]) + (b[2] + b[3])) + ((b[4] + b[5]) + (b[6] + b[7]));
+}
+
+void standalone_copies() {
+  static const bool entered = [] {
+    host_copy_enter();
+    return true;
+  }();
+  (void)entered;
 }
 
 int kspace_fix_launch(const double *src, double scale, double add, long long *dst,
@@ -563,11 +593,8 @@ int mdbas_nb_ewald_rec(int nAtom, const PBC *box, double alpha, double chargeCon
                       fz, 0, out);
   std::vector<double> hq(nAtom);
   MDB_CUDA(cudaMemcpy(hq.data(), q, sizeof(double) * nAtom, cudaMemcpyDeviceToHost));
-  double systq = 0., sumq2 = 0.;
-  for (int i = 0; i < nAtom; ++i) {
-    systq += hq[i];
-    sumq2 += hq[i] * hq[i];
-  }
+  double systq, sumq2;
+  charge_sums(nAtom, hq.data(), &systq, &sumq2);
   return ewald_run(nAtom, box, alpha, chargeConst, m1max, m2max, m3max, x, y, z, q, systq, sumq2,
                    fx, fy, fz, 0, out, static_cast<cudaStream_t>(stream));
 }

@@ -62,6 +62,10 @@ int ewald_launch(EwaldWork &c, int n, const PBC *box, double alpha, double charg
 int spme_launch(SpmeWork &c, int n, const PBC *box, double alpha, double chargeConst, int m1,
                 int m2, int m3, int nbsp, const double *x, const double *y, const double *z,
                 const double *q, double *fx, double *fy, double *fz, cudaStream_t s);
+// sum q and sum q^2 of the self and non-neutral terms.
+void charge_sums(int n, const double *q, double *systq, double *sumq2);
+// Registers the calls that belong to no engine with host_copy.cuh (once).
+void standalone_copies();
 // *dst = fixed point (2^-24) of scale * (*src) + add, on the device.
 int kspace_fix_launch(const double *src, double scale, double add, long long *dst,
                       cudaStream_t s);

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "host_copy.cuh"
 #include "list_ref.cuh"
 #include "pair_fp32.cuh"
 
@@ -1632,8 +1633,12 @@ int mdbas_nb_engine_get_positions(mdbas_nb_engine *e, double *x, double *y, doub
                                   int device_ptrs) {
   if (!e || !x || !y || !z) return MDBAS_NB_ERR_ARG;
   MDB_CUDA(cudaSetDevice(e->device));
-  const cudaMemcpyKind k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   const size_t bytes = sizeof(double) * (size_t)e->n;
+  if (!device_ptrs) {
+    const CopySpan out[3] = {{x, e->x.p, bytes}, {y, e->y.p, bytes}, {z, e->z.p, bytes}};
+    return copy_out(out, 3, e->stream);
+  }
+  const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
   MDB_CUDA(cudaMemcpyAsync(x, e->x.p, bytes, k, e->stream));
   MDB_CUDA(cudaMemcpyAsync(y, e->y.p, bytes, k, e->stream));
   MDB_CUDA(cudaMemcpyAsync(z, e->z.p, bytes, k, e->stream));
@@ -1646,9 +1651,13 @@ int mdbas_nb_engine_get_velocities(mdbas_nb_engine *e, double *vx, double *vy, d
   if (!e || !vx || !vy || !vz) return MDBAS_NB_ERR_ARG;
   if (!e->mdReady) return MDBAS_NB_ERR_STATE;
   MDB_CUDA(cudaSetDevice(e->device));
-  const cudaMemcpyKind k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   const size_t bytes = sizeof(double) * (size_t)e->n;
-  const double *v = e->mdV.as<double>();
+  double *v = e->mdV.as<double>();
+  if (!device_ptrs) {
+    const CopySpan3 out(vx, vy, vz, v, e->n);
+    return copy_out(out.s, 3, e->stream);
+  }
+  const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
   MDB_CUDA(cudaMemcpyAsync(vx, v, bytes, k, e->stream));
   MDB_CUDA(cudaMemcpyAsync(vy, v + e->n, bytes, k, e->stream));
   MDB_CUDA(cudaMemcpyAsync(vz, v + 2 * (size_t)e->n, bytes, k, e->stream));

@@ -78,11 +78,8 @@ int mdbas_nb_engine_set_kspace(mdbas_nb_engine *e, int kind, int m1, int m2, int
   // charge sums of the self and non-neutral terms (src/ewald.c:166-172)
   std::vector<double> hq(e->n);
   MDB_CUDA(cudaMemcpy(hq.data(), e->q.p, sizeof(double) * e->n, cudaMemcpyDeviceToHost));
-  double systq = 0., sumq2 = 0.;
-  for (int i = 0; i < e->n; ++i) {
-    systq += hq[i];
-    sumq2 += hq[i] * hq[i];
-  }
+  double systq, sumq2;
+  charge_sums(e->n, hq.data(), &systq, &sumq2);
   e->kspaceSystq = systq;
   e->kspaceSumq2 = sumq2;
   if (kind == 1 && !e->kEwald) e->kEwald = new EwaldWork();

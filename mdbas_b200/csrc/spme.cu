@@ -27,6 +27,7 @@
 #include <complex>
 #include <vector>
 
+#include "host_copy.cuh"
 #include "kspace.cuh"
 
 using namespace mdbas;
@@ -991,22 +992,13 @@ int spme_launch_impl(SpmeWork &c, int n, const PBC *box, double alpha, double ch
   return MDBAS_NB_OK;
 }
 
-int spme_run(int n, const PBC *box, double alpha, double chargeConst, int m1, int m2, int m3,
-             int nbsp, const double *x, const double *y, const double *z, const double *q,
-             double systq, double sumq2, double *fx, double *fy, double *fz, double out[8],
-             cudaStream_t s) {
-  SpmeWork &c = spme_ctx();
-  MDB_TRY(spme_launch_impl(c, n, box, alpha, chargeConst, m1, m2, m3, nbsp, x, y, z, q, fx, fy,
-                           fz, s));
-  const SpmeBox b = make_spme_box(box);
-  const double rvol = 6.283185307179586 / b.vol;
-  double *sums = c.sums.as<double>();
-  double h[16];
-  MDB_CUDA(cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, s));
-  MDB_CUDA(cudaStreamSynchronize(s));
+// Energy, virial and stress from the device sums h (src/spme.c:577-640).
+void spme_results(const PBC *box, double alpha, double chargeConst, double systq, double sumq2,
+                  const double *h, double out[8]) {
+  const double rvol = 6.283185307179586 / box->vol;
   const double eself = -chargeConst * alpha * sumq2 / kSqrtPi;
   const double enn = -(0.5 * 3.141592653589793 * chargeConst) *
-                     ((systq / alpha) * (systq / alpha) / b.vol);
+                     ((systq / alpha) * (systq / alpha) / box->vol);
   const double fact1 = rvol * chargeConst;
   const double erec = h[kSpmeEnergy];
   double st[6];
@@ -1019,6 +1011,19 @@ int spme_run(int n, const PBC *box, double alpha, double chargeConst, int m1, in
   out[0] = fact1 * erec + eself + enn;
   out[1] = -(st[0] + st[3] + st[5]);
   for (int k = 0; k < 6; ++k) out[2 + k] = st[k];
+}
+
+int spme_run(int n, const PBC *box, double alpha, double chargeConst, int m1, int m2, int m3,
+             int nbsp, const double *x, const double *y, const double *z, const double *q,
+             double systq, double sumq2, double *fx, double *fy, double *fz, double out[8],
+             cudaStream_t s) {
+  SpmeWork &c = spme_ctx();
+  MDB_TRY(spme_launch_impl(c, n, box, alpha, chargeConst, m1, m2, m3, nbsp, x, y, z, q, fx, fy,
+                           fz, s));
+  double h[16];
+  MDB_CUDA(cudaMemcpyAsync(h, c.sums.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+  MDB_CUDA(cudaStreamSynchronize(s));
+  spme_results(box, alpha, chargeConst, systq, sumq2, h, out);
   return MDBAS_NB_OK;
 }
 
@@ -1059,34 +1064,32 @@ int mdbas_nb_spme(int nAtom, const PBC *box, double alpha, double chargeConst, i
     MDB_CUDA(cudaMemcpy(hq.data(), q, sizeof(double) * nAtom, cudaMemcpyDeviceToHost));
     qh = hq.data();
   }
-  for (int i = 0; i < nAtom; ++i) {
-    systq += qh[i];
-    sumq2 += qh[i] * qh[i];
-  }
+  charge_sums(nAtom, qh, &systq, &sumq2);
   if (device_ptrs)
     return spme_run(nAtom, box, alpha, chargeConst, m1, m2, m3, nbsp, x, y, z, q, systq, sumq2,
                     fx, fy, fz, out, s);
   // host arrays: stage through device buffers; forces are added to the
   // caller's arrays
+  standalone_copies();
   MDB_TRY(c.xyzq.ensure(sizeof(double) * 4 * (size_t)nAtom));
   MDB_TRY(c.fout.ensure(sizeof(double) * 3 * (size_t)nAtom));
   double *d = c.xyzq.as<double>(), *f = c.fout.as<double>();
-  const size_t bytes = sizeof(double) * nAtom;
-  MDB_CUDA(cudaMemcpyAsync(d, x, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(d + nAtom, y, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(d + 2 * (size_t)nAtom, z, bytes, cudaMemcpyHostToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(d + 3 * (size_t)nAtom, q, bytes, cudaMemcpyHostToDevice, s));
+  const size_t bytes = sizeof(double) * (size_t)nAtom;
+  const CopySpan in[4] = {
+      {const_cast<double *>(x), d, bytes},
+      {const_cast<double *>(y), d + nAtom, bytes, false, true},
+      {const_cast<double *>(z), d + 2 * (size_t)nAtom, bytes, false, true},
+      {const_cast<double *>(q), d + 3 * (size_t)nAtom, bytes, false, true}};
+  MDB_TRY(copy_in(in, 4, s));
   MDB_CUDA(cudaMemsetAsync(f, 0, 3 * bytes, s));
-  MDB_TRY(spme_run(nAtom, box, alpha, chargeConst, m1, m2, m3, nbsp, d, d + nAtom,
-                   d + 2 * (size_t)nAtom, d + 3 * (size_t)nAtom, systq, sumq2, f, f + nAtom,
-                   f + 2 * (size_t)nAtom, out, s));
-  std::vector<double> hf(3 * (size_t)nAtom);
-  MDB_CUDA(cudaMemcpy(hf.data(), f, 3 * bytes, cudaMemcpyDeviceToHost));
-  for (int i = 0; i < nAtom; ++i) {
-    fx[i] += hf[i];
-    fy[i] += hf[nAtom + i];
-    fz[i] += hf[2 * (size_t)nAtom + i];
-  }
+  double h[16];
+  MDB_TRY(spme_launch_impl(c, nAtom, box, alpha, chargeConst, m1, m2, m3, nbsp, d, d + nAtom,
+                           d + 2 * (size_t)nAtom, d + 3 * (size_t)nAtom, f, f + nAtom,
+                           f + 2 * (size_t)nAtom, s));
+  const CopySpan3 f3(fx, fy, fz, f, nAtom, true);
+  const CopySpan o[4] = {f3.s[0], f3.s[1], f3.s[2], {h, c.sums.p, sizeof(h)}};
+  MDB_TRY(copy_out(o, 4, s));
+  spme_results(box, alpha, chargeConst, systq, sumq2, h, out);
   return MDBAS_NB_OK;
 }
 
