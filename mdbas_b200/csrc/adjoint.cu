@@ -104,8 +104,9 @@ __device__ __noinline__ RadialPair radial_general(const PairParams &p, double r2
 __device__ __forceinline__ RadialPair radial_fast(const PairParams &p, double r2, double rt,
                                                   double r, double x, double sig) {
   RadialPair o;
-  const double g = expm64(x * x);
-  const double A = p.chargeConst * 2.0 * p.alpha / kSqrtPi;
+  const EwaldConst ek(p);
+  const double g = expm64_product(ek.a2, ek.a2lo, r2);
+  const double A = p.chargeConst * ek.g0;
   o.c.e = p.chargeConst * (g * erfcx64(x)) * rt;
   o.c.d1 = -(o.c.e + A * g) * rt;
   o.c.d2 = -2.0 * o.c.d1 * rt + 2.0 * A * p.alpha * p.alpha * g;

@@ -134,24 +134,13 @@ __device__ __noinline__ PairTerms pair_ewald_slow(const PairParams &p, double qq
   return pair_general<true>(p, qq, veps, vsig, r2);
 }
 
-// 2 alpha / sqrt(pi), alpha^2 in two parts, and the switch's factor and
-// constant term.
-struct EwaldConst {
-  double g0, a2, a2lo, sw2, swc;
-};
-
 // The same Ewald pair with the forms of real64.cuh; the caller has checked
 // that r2 and alpha r lie in their range.
-//
-// exp takes alpha^2 r^2, from a product in two parts (a2 + a2lo is alpha^2 to
-// twice the precision): a rounded x^2 would put an error of x^2 ulps on it.
 __device__ __forceinline__ PairTerms pair_ewald_fast(const PairParams &p, const EwaldConst &k,
                                                      double qq, double veps, double vsig,
                                                      double r2, double rt, double x) {
   PairTerms o;
-  const double u = k.a2 * r2;
-  const double g1 = expm64(u);
-  const double g = fma(-g1, fma(k.a2, r2, fma(k.a2lo, r2, -u)), g1);
+  const double g = expm64_product(k.a2, k.a2lo, r2);
   o.eel = qq * (g * erfcx64(x)) * rt;
   o.wel = -fma(k.g0 * qq, g, o.eel);
   o.evdw = o.wvdw = 0.;
@@ -220,12 +209,7 @@ k_pairs_fp64(int n, DevBox b, PairParams p, HalfList hl, const double *__restric
   __shared__ RowQueue queues[kRowWarps];
   __shared__ double red[5][kRowWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  EwaldConst ek;
-  ek.g0 = 2.0 * p.alpha / kSqrtPi;
-  ek.a2 = p.alpha * p.alpha;
-  ek.a2lo = fma(p.alpha, p.alpha, -ek.a2);
-  ek.sw2 = p.switch2;
-  ek.swc = p.cutOff2 - 3. * p.cutOn2;
+  const EwaldConst ek(p);
   double eel = 0., evdw = 0., virel = 0., virvdw = 0.;
   int npair = 0;
   double qi, ei, si, fxi, fyi, fzi;

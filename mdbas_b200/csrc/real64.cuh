@@ -80,4 +80,21 @@ __device__ __forceinline__ double expm64(double u) {
   return __hiloint2double(__double2hiint(p) + (__double2loint(m) << 20), __double2loint(p));
 }
 
+// exp(-(a2 + a2lo) r2) from a product in two parts (a2 + a2lo is alpha^2 to
+// twice the precision): a rounded x^2 would put an error of x^2 ulps on it.
+__device__ __forceinline__ double expm64_product(double a2, double a2lo, double r2) {
+  const double u = a2 * r2;
+  const double g = expm64(u);
+  return fma(-g, fma(a2, r2, fma(a2lo, r2, -u)), g);
+}
+
+// 2 alpha / sqrt(pi), alpha^2 in two parts, and the switch's factor and
+// constant term.
+struct EwaldConst {
+  double g0, a2, a2lo, sw2, swc;
+  __device__ __forceinline__ explicit EwaldConst(const PairParams &p)
+      : g0(2.0 * p.alpha / kSqrtPi), a2(p.alpha * p.alpha), a2lo(fma(p.alpha, p.alpha, -a2)),
+        sw2(p.switch2), swc(p.cutOff2 - 3. * p.cutOn2) {}
+};
+
 }  // namespace mdbas
