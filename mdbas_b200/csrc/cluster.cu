@@ -35,6 +35,10 @@ namespace mdbas {
 namespace {
 
 constexpr int kSearchThreads = 128;
+// Most atoms of the search's block-per-cluster form: the build with it and
+// with a warp per cluster takes 67 and 85 us at 2,001 atoms, 70 and 92 at
+// 3,000, 82 and 93 at 9,000, 91 and 97 at 12,000, but 131 and 114 at 24,000.
+constexpr int kTeamAtoms = 12000;
 constexpr int kBufCap = 64;
 
 __device__ __forceinline__ double wrap_pos(double v, double L, double invL) {
@@ -812,6 +816,14 @@ k_col_ztab(int nCols, const ClusterGeom *__restrict__ geoms, const int *__restri
 // the upper triangle of atom pairs).
 // (at most 96 registers and ~34 KB of shared memory per block: five blocks
 // of four warps per SM)
+//
+// TEAM: the block's four warps share one cluster, for systems with so few
+// clusters that the search is one warp's serial time (the build of 3,000
+// atoms: 92 -> 70 us).  Each warp lists the columns for itself and
+// tests every fourth round of candidates; a round's survivors go to the shared
+// buffer behind those of the rounds before it, and every 32 of them are one
+// warp's flush: the same work items as one warp makes.
+template <bool TEAM>
 __global__ void __launch_bounds__(kSearchThreads, 5)
 k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geoms,
          const DevBox *__restrict__ boxes, const int *__restrict__ clusterRep,
@@ -824,9 +836,13 @@ k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geom
          const int *__restrict__ hmaxBits, const float4 *__restrict__ xq,
          const double *__restrict__ px, const double *__restrict__ py,
          const double *__restrict__ pz, const SearchOut o) {
-  __shared__ WarpBuf bufs[kSearchThreads / 32];
-  const int lane = threadIdx.x & 31;
-  const int ci = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  constexpr int kWarps = kSearchThreads / 32;
+  constexpr int kTeam = TEAM ? kWarps : 1;  // warps per cluster
+  __shared__ WarpBuf bufs[kWarps];
+  __shared__ int teamJ[TEAM ? 64 * kWarps : 1], teamCode[TEAM ? 64 * kWarps : 1];
+  __shared__ int teamCnt[kWarps];
+  const int lane = threadIdx.x & 31, sub = TEAM ? threadIdx.x >> 5 : 0;
+  const int ci = TEAM ? blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nClusters = *nSlotsDev >> 3;
   if (ci >= nClusters) return;
   WarpBuf &B = bufs[threadIdx.x >> 5];
@@ -979,9 +995,15 @@ k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geom
     const int total = __shfl_sync(0xffffffffu, incl, 31);
     __syncwarp();
     int k0 = 0;  // the listed range holding flat index b0
-    for (int b0 = 0; b0 < total; b0 += 32) {
+    for (int r0 = 0; r0 < total; r0 += 32 * kTeam) {
+      const int b0 = r0 + 32 * sub;
       const int t = b0 + lane;
       const bool valid = t < total;
+      if (TEAM) {  // the range holding b0 (the last one when there is none)
+        k0 = 0;
+        for (int step = 128; step > 0; step >>= 1)
+          if (k0 + step < ncol && B.rpre[k0 + step] <= b0) k0 += step;
+      }
       int cj = 0, sx = 0, sy = 0, sz = 0;
       float4 oj = make_float4(0.f, 0.f, 1e30f, 0.f);
       float4 hj = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1015,6 +1037,38 @@ k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geom
       const bool half_ok = (cj > ci) || (cj == ci && (sidx == 13 || positive));
       const bool ok = valid && half_ok && (gxx * gxx + gyy * gyy + gzz * gzz <= rlist2);
       const unsigned m = __ballot_sync(0xffffffffu, ok);
+      if (TEAM) {
+        if (lane == 0) teamCnt[sub] = __popc(m);
+        __syncthreads();
+        int pos = cnt + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+          const int c = teamCnt[w];
+          if (w < sub) pos += c;
+          cnt += c;
+        }
+        if (ok) {
+          teamJ[pos] = cj;
+          teamCode[pos] = sidx | ((int)hj.w << 8);
+        }
+        __syncthreads();
+        if (cnt >= kItemMax * kWarps) {
+          B.j[lane] = teamJ[kItemMax * sub + lane];
+          B.code[lane] = teamCode[kItemMax * sub + lane];
+          __syncwarp();
+          flush_item(B, kItemMax, ci, lane, xq, g, box, nreal_i, pcLo, pcHi, fimask, exclFlat,
+                     slotOf, slotAtom, frozen, px, py, pz, origin, o);
+          // what is left (fewer than one entry per thread) to the front
+          const int rj = teamJ[kItemMax * kWarps + threadIdx.x];
+          const int rc = teamCode[kItemMax * kWarps + threadIdx.x];
+          __syncthreads();
+          teamJ[threadIdx.x] = rj;
+          teamCode[threadIdx.x] = rc;
+          cnt -= kItemMax * kWarps;
+          __syncthreads();
+        }
+        continue;
+      }
       if (ok) {
         const int pos = cnt + __popc(m & ((1u << lane) - 1u));
         B.j[pos] = cj;
@@ -1038,6 +1092,15 @@ k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geom
     ncol = 0;
     __syncwarp();
   }
+  if (TEAM) {
+    // the groups that are left, one warp each
+    cnt = min(max(cnt - kItemMax * sub, 0), kItemMax);
+    if (lane < cnt) {
+      B.j[lane] = teamJ[kItemMax * sub + lane];
+      B.code[lane] = teamCode[kItemMax * sub + lane];
+    }
+    __syncwarp();
+  }
   if (cnt > 0)
     flush_item(B, cnt, ci, lane, xq, g, box, nreal_i, pcLo, pcHi, fimask, exclFlat, slotOf,
                slotAtom, frozen, px, py, pz, origin, o);
@@ -1059,7 +1122,11 @@ k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geom
       atomicAdd(reinterpret_cast<unsigned long long *>(o.hcounters + 4),
                 (unsigned long long)B.tally[3]);
     }
-    // The warp that finishes last (counters[7] counts the finished ones)
+    __threadfence();
+  }
+  if (TEAM) __syncthreads();  // the team's sums are in before it counts as finished
+  if (lane == 0 && sub == 0) {
+    // The cluster that finishes last (counters[7] counts the finished ones)
     // writes the readers' counts: entries kept (counters[5]) and inner halves
     // written (hcounters[6]); both lists have the packed counter's item count
     // (items << 40 | entries taken, counters[4]).  For a build that does not
@@ -1068,7 +1135,6 @@ k_search(const int *__restrict__ nSlotsDev, const ClusterGeom *__restrict__ geom
     // and some items were never written), so the counts of both lists are
     // zeroed and the pair kernels that follow in the same stream (or graph)
     // see an empty list until the host rebuilds with room.
-    __threadfence();
     const unsigned long long done =
         atomicAdd(reinterpret_cast<unsigned long long *>(o.counters + 7), 1ull);
     if (done + 1ull == (unsigned long long)nClusters) {
@@ -1491,8 +1557,11 @@ int cluster_build(ClusterWork &w, int n, int nRep, const DevBox *boxes, const in
     o.rin2 = rin2;
     o.sticky = sync ? nullptr : w.sticky.as<long long>();
   if (w.timeStages) MDB_CUDA(cudaEventRecord(w.stageEv[5], s));
-    MDB_LAUNCH(k_search, grid_for((long long)w.clCap * 32, kSearchThreads), kSearchThreads, 0, s,
-               w.nSlotsDev(), gd, w.boxes.as<DevBox>(), w.clusterRepDev(), w.colOff.as<int>(),
+    const bool team = n <= kTeamAtoms;
+    const auto search = team ? k_search<true> : k_search<false>;
+    MDB_LAUNCH(search, team ? w.clCap : grid_for((long long)w.clCap * 32, kSearchThreads),
+               kSearchThreads, 0, s, w.nSlotsDev(), gd, w.boxes.as<DevBox>(), w.clusterRepDev(),
+               w.colOff.as<int>(),
                w.zTab.as<int>(), w.clusterXY.as<int>(),
                w.origin.as<double4>(), w.originF.as<float4>(), w.half.as<float4>(),
                w.slotAtom.as<int>(), w.slotOf.as<int>(), frozen, exclStart, exclFlat,
