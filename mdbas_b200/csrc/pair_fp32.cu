@@ -984,8 +984,13 @@ k_pair_half(const long long *__restrict__ counters, const int4 *__restrict__ ite
 // for the range check (a NaN shows up in the i forces, checked per item),
 // the per-lane 64-bit energy sums live in shared memory, and warps take items
 // from a counter.  Forces and energies equal k_pair_half's bit for bit.
+// Three blocks per SM with the step loop unrolled by four (80 registers): two
+// steps' loads and exponentials in flight are worth more than the fourth
+// block.  Blocks x unroll, full list of 96,000 atoms: 4x1 317 us, 4x2 317,
+// 3x1 316, 3x2 308, 3x4 306, 2x4 333; 10^6 atoms 2,930 -> 2,840 us, its exact
+// inner list 2,285 -> 2,218; 3,000 atoms 55 -> 52.
 template <bool VDW, bool INNER, bool EXACT>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 3)
 k_pair_half_lean(const long long *__restrict__ counters, const int4 *__restrict__ items,
             const void *__restrict__ entriesV, const void *__restrict__ masksV,
             const float4 *__restrict__ xq, const float2 *__restrict__ lj, PairConstF c,
@@ -1098,6 +1103,7 @@ k_pair_half_lean(const long long *__restrict__ counters, const int4 *__restrict_
       __syncwarp();
       const float4 *__restrict__ jdl = S.jd[up ? 1 : 0];
       const int4 *__restrict__ mjl = S.mj[up ? 1 : 0];
+#pragma unroll 4
       for (int k = 0; k < nIt; ++k) {
         // this lane's two pairs: .x with the half it keeps in the reduction
         const float4 p0 = jdl[(k * 4 + jl) * 3], p1 = jdl[(k * 4 + jl) * 3 + 1];
