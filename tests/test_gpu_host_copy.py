@@ -68,3 +68,14 @@ def test_threads(gpu):
     for t in ts:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("n", [1, 21845, 21846, 65536, 65537, 200003, 700001])
+def test_round_trip_through_slots(gpu, n):
+    """Past the results that are copied before the slots exist."""
+    s = _atoms(n)
+    e = _engine(s)
+    for _ in range(12):
+        for a, b in zip(e.positions(), (s.x, s.y, s.z)):
+            assert np.array_equal(a, b)
+    e.close()
