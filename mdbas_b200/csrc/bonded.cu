@@ -351,8 +351,8 @@ int bonded_set(BondedTerms &t, int nAtom, const int count[KIND_COUNT],
   return MDBAS_NB_OK;
 }
 
-int bonded_eval(BondedTerms &t, const DevBox *boxes, const int *atomRep, const double *x,
-                const double *y, const double *z, double *f, cudaStream_t s) {
+int bonded_terms(BondedTerms &t, const DevBox *boxes, const int *atomRep, const double *x,
+                 const double *y, const double *z, cudaStream_t s) {
   const int nt = t.nTerms();
   if (nt == 0 || t.nAtom == 0) return MDBAS_NB_OK;
   BondedArgs a;
@@ -369,10 +369,21 @@ int bonded_eval(BondedTerms &t, const DevBox *boxes, const int *atomRep, const d
   const int nb = grid_for(nt, kBondedBlock);
   double *c = t.contrib.as<double>(), *part = t.part.as<double>();
   MDB_LAUNCH(k_bonded_terms, nb, kBondedBlock, 0, s, a, boxes, atomRep, x, y, z, c, part);
-  MDB_LAUNCH(k_bonded_gather, grid_for(t.nAtom, 256), 256, 0, s, t.nAtom,
-             t.atomStart.as<int>(), t.atomSlot.as<int>(), c, a.nSlots, f);
   MDB_LAUNCH(k_bonded_finish, 1, 256, 0, s, nb, part, t.sums.as<double>());
   return MDBAS_NB_OK;
+}
+
+int bonded_add(BondedTerms &t, double *f, cudaStream_t s) {
+  if (t.nTerms() == 0 || t.nAtom == 0) return MDBAS_NB_OK;
+  MDB_LAUNCH(k_bonded_gather, grid_for(t.nAtom, 256), 256, 0, s, t.nAtom,
+             t.atomStart.as<int>(), t.atomSlot.as<int>(), t.contrib.as<double>(), t.nSlots(), f);
+  return MDBAS_NB_OK;
+}
+
+int bonded_eval(BondedTerms &t, const DevBox *boxes, const int *atomRep, const double *x,
+                const double *y, const double *z, double *f, cudaStream_t s) {
+  MDB_TRY(bonded_terms(t, boxes, atomRep, x, y, z, s));
+  return bonded_add(t, f, s);
 }
 
 }  // namespace mdbas

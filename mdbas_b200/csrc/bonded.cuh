@@ -42,10 +42,14 @@ struct BondedTerms {
 // atoms and build the slot lists.  Every atom index must lie in [0, nAtom).
 int bonded_set(BondedTerms &t, int nAtom, const int count[KIND_COUNT],
                const void *const terms[KIND_COUNT], cudaStream_t s);
-// Forces added in place to f (3 * nAtom: x block, y block, z block, device)
-// and the energy sums into t.sums, at positions x, y, z (device).  boxes /
-// atomRep: the per-replica boxes and atom -> replica map (atomRep may be null
-// for a single box).
+// Every term's forces into its slots and the energy sums into t.sums, at
+// positions x, y, z (device).  boxes / atomRep: the per-replica boxes and
+// atom -> replica map (atomRep may be null for a single box).
+int bonded_terms(BondedTerms &t, const DevBox *boxes, const int *atomRep, const double *x,
+                 const double *y, const double *z, cudaStream_t s);
+// The slots added in place to f (3 * nAtom: x block, y block, z block, device).
+int bonded_add(BondedTerms &t, double *f, cudaStream_t s);
+// Both.
 int bonded_eval(BondedTerms &t, const DevBox *boxes, const int *atomRep, const double *x,
                 const double *y, const double *z, double *f, cudaStream_t s);
 

@@ -104,6 +104,9 @@ struct mdbas_nb_engine {
   cudaGraph_t mdGraph = nullptr;
   cudaGraphExec_t mdExec = nullptr;
   cudaStream_t mdCapStream = nullptr, mdSideStream = nullptr;
+  // branches of the captured step (md.cu: MdBranch) and their fork/join events
+  cudaStream_t mdBranch[3] = {};
+  cudaEvent_t mdForkEv = nullptr, mdJoinEv[3] = {};
   mdbas::DBuf mdRows, mdSnap;
 };
 
@@ -120,9 +123,11 @@ struct LaunchScope {
 int engine_check_device(int device);
 // Releases the dynamics graph and its streams (md.cu).
 void md_release(mdbas_nb_engine *e);
-// Reciprocal forces added to f (3n, caller order) and the reciprocal plus
-// non-neutral energy into kspaceFix (md_kspace.cu); no-op when off.
-int md_kspace(mdbas_nb_engine *e, double *f, cudaStream_t s);
+// Reciprocal space at the engine's positions (md_kspace.cu): the forces into
+// its own buffers and the reciprocal plus non-neutral energy into kspaceFix;
+// the forces added to f (3n, caller order).  No-ops when off.
+int md_kspace_terms(mdbas_nb_engine *e, cudaStream_t s);
+int md_kspace_add(mdbas_nb_engine *e, double *f, cudaStream_t s);
 // Settle a pending build (see buildPending): read its error bits; on an
 // overflowing list build again with room, synchronously, and redo the
 // evaluation if one ran on the empty list; non-finite positions are an error.

@@ -414,7 +414,6 @@ int ewald_launch_impl(EwaldWork &c, int n, const PBC *box, double alpha, double 
   MDB_TRY(c.sums.ensure(sizeof(double) * 8));
   const double rVol = kTwoPi / box->vol;
   const double fact1 = 2.0 * rVol * chargeConst;
-  const double fact0 = 2.0 * fact1;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int parts = 0;
@@ -456,10 +455,9 @@ int ewald_launch_impl(EwaldWork &c, int n, const PBC *box, double alpha, double 
                kl.rowBase.as<double4>(), kTwoPi * box->w1, kTwoPi * box->w2, kTwoPi * box->w3,
                c.S.as<double2>(), tab, q, c.pf.as<double>());
   }
-  MDB_LAUNCH(k_ewald_add, dim3(grid_for(n, 256), 3), 256, 0, s, n, parts, c.pf.as<double>(), fact0,
-             scaleInput, fx, fy, fz);
+  c.parts = parts;
   c.fact1 = fact1;
-  return MDBAS_NB_OK;
+  return fx ? ewald_add(c, n, fx, fy, fz, scaleInput, s) : MDBAS_NB_OK;
 }
 
 // out[0] = energy (reciprocal + self + non-neutral), out[1] = virial,
@@ -535,6 +533,13 @@ __global__ void k_kspace_fix(const double *__restrict__ src, double scale, doubl
 }
 
 }  // namespace
+
+int ewald_add(EwaldWork &c, int n, double *fx, double *fy, double *fz, int scaleInput,
+              cudaStream_t s) {
+  MDB_LAUNCH(k_ewald_add, dim3(grid_for(n, 256), 3), 256, 0, s, n, c.parts, c.pf.as<double>(),
+             2.0 * c.fact1, scaleInput, fx, fy, fz);
+  return MDBAS_NB_OK;
+}
 
 int ewald_launch(EwaldWork &c, int n, const PBC *box, double alpha, double chargeConst, int M1,
                  int M2, int M3, const double *x, const double *y, const double *z,

@@ -21,6 +21,7 @@ struct EwaldWork {
   EwaldKList kl;
   int device = -1;
   DBuf part, S, bpart, sums, tab, pf, done, xyzq, f;
+  int parts = 0;      // of the last launch's forces (pf)
   double fact1 = 0.;  // 2 (2 pi / V) C of the last launch
 };
 
@@ -62,6 +63,10 @@ int ewald_launch(EwaldWork &c, int n, const PBC *box, double alpha, double charg
 int spme_launch(SpmeWork &c, int n, const PBC *box, double alpha, double chargeConst, int m1,
                 int m2, int m3, int nbsp, const double *x, const double *y, const double *z,
                 const double *q, double *fx, double *fy, double *fz, cudaStream_t s);
+// Both without the additions when fx is null; these make them.
+int ewald_add(EwaldWork &c, int n, double *fx, double *fy, double *fz, int scaleInput,
+              cudaStream_t s);
+int spme_add(SpmeWork &c, int n, double *fx, double *fy, double *fz, cudaStream_t s);
 // sum q and sum q^2 of the self and non-neutral terms.
 void charge_sums(int n, const double *q, double *systq, double *sumq2);
 // Registers the calls that belong to no engine with host_copy.cuh (once).

@@ -827,10 +827,17 @@ const long long *md_kspace_fix(const mdbas_nb_engine *e) {
   return e->kspaceKind != 0 ? e->kspaceFix.as<long long>() : nullptr;
 }
 
+int md_bonded_terms(mdbas_nb_engine *e, cudaStream_t s) {
+  if (e->bonded.nTerms() == 0) return MDBAS_NB_OK;
+  return bonded_terms(e->bonded, BOXES(e), e->x.as<double>(), e->y.as<double>(),
+                      e->z.as<double>(), s);
+}
+
 // FP64 forces of the last compute, caller order, into e->mdF (3n); then the
-// bonded terms in MDBas's order (energy(), src/energy.c:167-190) and the
-// frozen atoms (freeze_atoms, src/energy.c:198-201).
-int md_forces(mdbas_nb_engine *e, cudaStream_t s) {
+// reciprocal forces and bonded terms (of md_kspace_terms and md_bonded_terms)
+// in MDBas's order (energy(), src/energy.c:167-190) and the frozen atoms
+// (freeze_atoms, src/energy.c:198-201).
+int md_sum_forces(mdbas_nb_engine *e, cudaStream_t s) {
   const int n = e->n;
   double *f = e->mdF.as<double>();
   if (e->cfg.precision == 0) {
@@ -839,14 +846,18 @@ int md_forces(mdbas_nb_engine *e, cudaStream_t s) {
   } else {
     MDB_TRY(forces_out_launch(e->cl, n, 0, f, f + n, f + 2 * (size_t)n, s));
   }
-  MDB_TRY(md_kspace(e, f, s));
-  if (e->bonded.nTerms() > 0)
-    MDB_TRY(bonded_eval(e->bonded, BOXES(e), e->x.as<double>(), e->y.as<double>(),
-                        e->z.as<double>(), f, s));
+  MDB_TRY(md_kspace_add(e, f, s));
+  MDB_TRY(bonded_add(e->bonded, f, s));
   if (e->hasFrozen)
     MDB_LAUNCH(k_freeze, grid_for(n, 256), 256, 0, s, n, e->frozen.as<int>(), f,
                e->mdV.as<double>());
   return MDBAS_NB_OK;
+}
+
+int md_forces(mdbas_nb_engine *e, cudaStream_t s) {
+  MDB_TRY(md_kspace_terms(e, s));
+  MDB_TRY(md_bonded_terms(e, s));
+  return md_sum_forces(e, s);
 }
 
 int md_save_build_positions(mdbas_nb_engine *e, cudaStream_t s) {
@@ -949,18 +960,55 @@ int md_prune_sync(mdbas_nb_engine *e) {
   return MDBAS_NB_OK;
 }
 
-// Nonbonded forces of the cluster form with no host interaction, on the
-// current layout (refreshed by the caller): evaluate, convert to caller order.
+// The branches of a captured step.  Reciprocal space and the bonded terms need
+// the new positions only, and run beside the list update and the pair kernel;
+// the exclusion correction adds into the pair kernel's fixed-point words.  The
+// pair kernel of 10,000 atoms leaves most of the chip idle for its 52 us, and
+// the 16 kernels of its SPME take 105: a step of flexible chains with SPME
+// 196 -> 160 us; of 96,000 atoms of water (the exclusions' 11 us) 441 -> 434.
+enum MdBranch { BR_KSPACE = 0, BR_BONDED = 1, BR_EXCL = 2 };
+
+int md_fork(mdbas_nb_engine *e, MdBranch b, cudaStream_t s) {
+  MDB_CUDA(cudaEventRecord(e->mdForkEv, s));
+  MDB_CUDA(cudaStreamWaitEvent(e->mdBranch[b], e->mdForkEv, 0));
+  return MDBAS_NB_OK;
+}
+
+int md_join(mdbas_nb_engine *e, MdBranch b, cudaStream_t s) {
+  MDB_CUDA(cudaEventRecord(e->mdJoinEv[b], e->mdBranch[b]));
+  MDB_CUDA(cudaStreamWaitEvent(s, e->mdJoinEv[b], 0));
+  return MDBAS_NB_OK;
+}
+
+// The captured step's branches that start at the new positions.
+int md_fork_terms(mdbas_nb_engine *e, cudaStream_t s) {
+  if (e->kspaceKind != 0) {
+    MDB_TRY(md_fork(e, BR_KSPACE, s));
+    MDB_TRY(md_kspace_terms(e, e->mdBranch[BR_KSPACE]));
+  }
+  if (e->bonded.nTerms() > 0) {
+    MDB_TRY(md_fork(e, BR_BONDED, s));
+    MDB_TRY(md_bonded_terms(e, e->mdBranch[BR_BONDED]));
+  }
+  return MDBAS_NB_OK;
+}
+
+// Forces of a captured step on the current layout (refreshed by the caller):
+// evaluate, join the branches, convert to caller order.
 int md_forces_cluster(mdbas_nb_engine *e, cudaStream_t s) {
   ClusterWork &w = e->cl;
   const int n = e->n;
   MDB_CUDA(cudaMemsetAsync(w.facc.p, 0, sizeof(long long) * 3 * (size_t)w.slotCap, s));
   MDB_CUDA(cudaMemsetAsync(w.acc.p, 0, sizeof(long long) * ACC_COUNT, s));
-  MDB_TRY(pair_fp32_launch(w, e->pp, e->grid, e->block, s, e->variant));
+  MDB_TRY(md_fork(e, BR_EXCL, s));
   MDB_TRY(excl_fix_launch(w, n, e->pp, e->exclStartSym.as<int>(), e->exclFlatSym.as<int>(),
                           e->x.as<double>(), e->y.as<double>(), e->z.as<double>(),
-                          e->q.as<double>(), s));
-  return md_forces(e, s);
+                          e->q.as<double>(), e->mdBranch[BR_EXCL]));
+  MDB_TRY(pair_fp32_launch(w, e->pp, e->grid, e->block, s, e->variant));
+  MDB_TRY(md_join(e, BR_EXCL, s));
+  if (e->kspaceKind != 0) MDB_TRY(md_join(e, BR_KSPACE, s));
+  if (e->bonded.nTerms() > 0) MDB_TRY(md_join(e, BR_BONDED, s));
+  return md_sum_forces(e, s);
 }
 
 int md_refresh_cluster(mdbas_nb_engine *e, cudaStream_t s) {
@@ -1123,6 +1171,7 @@ int md_capture_steps(mdbas_nb_engine *e, int K, double tauT, double kinTemp0,
   for (int k = 0; k < K; ++k) {
     g_launch_counter = &cc.main;
     MDB_TRY(md_stage1(e, cs));
+    MDB_TRY(md_fork_terms(e, cs));
     // the rebuild and prune decisions, on the device
     cudaStreamCaptureStatus cst;
     cudaGraph_t capG = nullptr;
@@ -1173,6 +1222,11 @@ int md_capture(mdbas_nb_engine *e, int K, double targetTemp, double tauT, double
     MDB_CUDA(cudaStreamCreateWithFlags(&e->mdCapStream, cudaStreamNonBlocking));
   if (!e->mdSideStream)
     MDB_CUDA(cudaStreamCreateWithFlags(&e->mdSideStream, cudaStreamNonBlocking));
+  for (cudaStream_t &b : e->mdBranch)
+    if (!b) MDB_CUDA(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
+  if (!e->mdForkEv) MDB_CUDA(cudaEventCreateWithFlags(&e->mdForkEv, cudaEventDisableTiming));
+  for (cudaEvent_t &ev : e->mdJoinEv)
+    if (!ev) MDB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   MDB_TRY(e->mdRows.ensure(sizeof(long long) * kRowWords * (size_t)K));
   // everything the capture reads from the host must be final: finish the
   // engine stream's work first
@@ -1316,6 +1370,16 @@ void mdbas::md_release(mdbas_nb_engine *e) {
   if (e->mdCapStream) cudaStreamDestroy(e->mdCapStream);
   if (e->mdSideStream) cudaStreamDestroy(e->mdSideStream);
   e->mdCapStream = e->mdSideStream = nullptr;
+  for (cudaStream_t &b : e->mdBranch) {
+    if (b) cudaStreamDestroy(b);
+    b = nullptr;
+  }
+  for (cudaEvent_t &ev : e->mdJoinEv) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
+  }
+  if (e->mdForkEv) cudaEventDestroy(e->mdForkEv);
+  e->mdForkEv = nullptr;
 }
 
 extern "C" {

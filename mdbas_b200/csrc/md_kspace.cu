@@ -24,30 +24,34 @@ double kspace_enn(const mdbas_nb_engine *e) {
          ((e->kspaceSystq / a) * (e->kspaceSystq / a) / e->hostBox.vol);
 }
 
-int kspace_launch(mdbas_nb_engine *e, double *f, cudaStream_t s) {
+}  // namespace
+
+int mdbas::md_kspace_terms(mdbas_nb_engine *e, cudaStream_t s) {
+  if (e->kspaceKind == 0) return MDBAS_NB_OK;
   const int n = e->n;
   const double *x = e->x.as<double>(), *y = e->y.as<double>(), *z = e->z.as<double>();
   const double *q = e->q.as<double>();
-  double *fy = f + n, *fz = f + 2 * (size_t)n;
+  double *const none = nullptr;
   if (e->kspaceKind == 1) {
     MDB_TRY(ewald_launch(*e->kEwald, n, &e->hostBox, e->cfg.alpha, e->cfg.chargeConst,
-                         e->kspaceM[0], e->kspaceM[1], e->kspaceM[2], x, y, z, q, f, fy, fz, 0,
-                         s));
+                         e->kspaceM[0], e->kspaceM[1], e->kspaceM[2], x, y, z, q, none, none,
+                         none, 0, s));
     return kspace_fix_launch(e->kEwald->sums.as<double>(), e->kEwald->fact1, kspace_enn(e),
                              e->kspaceFix.as<long long>(), s);
   }
   MDB_TRY(spme_launch(*e->kSpme, n, &e->hostBox, e->cfg.alpha, e->cfg.chargeConst,
-                      e->kspaceM[0], e->kspaceM[1], e->kspaceM[2], e->kspaceOrder, x, y, z, q, f,
-                      fy, fz, s));
+                      e->kspaceM[0], e->kspaceM[1], e->kspaceM[2], e->kspaceOrder, x, y, z, q, none,
+                      none, none, s));
   return kspace_fix_launch(e->kSpme->sums.as<double>() + kSpmeEnergy, e->kSpme->f1, kspace_enn(e),
                            e->kspaceFix.as<long long>(), s);
 }
 
-}  // namespace
-
-int mdbas::md_kspace(mdbas_nb_engine *e, double *f, cudaStream_t s) {
-  if (e->kspaceKind == 0) return MDBAS_NB_OK;
-  return kspace_launch(e, f, s);
+int mdbas::md_kspace_add(mdbas_nb_engine *e, double *f, cudaStream_t s) {
+  const int n = e->n;
+  double *fy = f + n, *fz = f + 2 * (size_t)n;
+  return e->kspaceKind == 1   ? ewald_add(*e->kEwald, n, f, fy, fz, 0, s)
+         : e->kspaceKind == 2 ? spme_add(*e->kSpme, n, f, fy, fz, s)
+                              : MDBAS_NB_OK;
 }
 
 void mdbas::kspace_release(mdbas_nb_engine *e) {
@@ -91,7 +95,8 @@ int mdbas_nb_engine_set_kspace(mdbas_nb_engine *e, int kind, int m1, int m2, int
   if (e->posSet) {
     LaunchScope ls(e);
     MDB_CUDA(cudaMemsetAsync(e->kspaceF.p, 0, sizeof(double) * 3 * (size_t)e->n, e->stream));
-    MDB_TRY(kspace_launch(e, e->kspaceF.as<double>(), e->stream));
+    MDB_TRY(md_kspace_terms(e, e->stream));
+    MDB_TRY(md_kspace_add(e, e->kspaceF.as<double>(), e->stream));
     MDB_CUDA(cudaStreamSynchronize(e->stream));
   }
   return MDBAS_NB_OK;
@@ -108,7 +113,8 @@ int mdbas_nb_engine_kspace(mdbas_nb_engine *e, double *fx, double *fy, double *f
   const size_t bytes = sizeof(double) * (size_t)n;
   double *f = e->kspaceF.as<double>();
   MDB_CUDA(cudaMemsetAsync(f, 0, 3 * bytes, s));
-  MDB_TRY(kspace_launch(e, f, s));
+  MDB_TRY(md_kspace_terms(e, s));
+  MDB_TRY(md_kspace_add(e, f, s));
   // energy: the reciprocal and non-neutral terms plus the self term
   double sums[10];
   const double *dsums = e->kspaceKind == 1 ? e->kEwald->sums.as<double>()

@@ -986,10 +986,8 @@ int spme_launch_impl(SpmeWork &c, int n, const PBC *box, double alpha, double ch
                group, b, -2.0 * rvol * chargeConst, q, c.spl.as<double>(), c.cell.as<int>(), grid,
                c.fr.as<double>(), part, done, sums + 7);
   }
-  MDB_LAUNCH(k_spme_add, grid_for(n, 256), 256, 0, s, n, c.fr.as<double>(), sums + 7, fx, fy,
-             fz);
   c.f1 = rvol * chargeConst;
-  return MDBAS_NB_OK;
+  return fx ? spme_add(c, n, fx, fy, fz, s) : MDBAS_NB_OK;
 }
 
 // Energy, virial and stress from the device sums h (src/spme.c:577-640).
@@ -1036,6 +1034,12 @@ int check_grid(int m1, int m2, int m3, int nbsp) {
 int nint_h(double x) { return (x >= 0.) ? (int)(x + 0.5) : (int)(x - 0.5); }
 
 }  // namespace
+
+int mdbas::spme_add(SpmeWork &c, int n, double *fx, double *fy, double *fz, cudaStream_t s) {
+  MDB_LAUNCH(k_spme_add, grid_for(n, 256), 256, 0, s, n, c.fr.as<double>(),
+             c.sums.as<double>() + 7, fx, fy, fz);
+  return MDBAS_NB_OK;
+}
 
 int mdbas::spme_launch(SpmeWork &c, int n, const PBC *box, double alpha, double chargeConst,
                        int m1, int m2, int m3, int nbsp, const double *x, const double *y,
