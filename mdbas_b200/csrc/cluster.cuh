@@ -188,5 +188,7 @@ int cluster_read_counts(ClusterWork &w, cudaStream_t s);
 // Refresh xq from the current FP64 positions (list kept).
 int cluster_refresh(ClusterWork &w, const double *x, const double *y, const double *z,
                     const double *q, double sqrtC, cudaStream_t s);
+// Zero the force and energy words (facc, acc) of an evaluation.
+int cluster_clear(ClusterWork &w, cudaStream_t s);
 
 }  // namespace mdbas

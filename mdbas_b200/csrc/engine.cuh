@@ -94,7 +94,7 @@ struct mdbas_nb_engine {
   int mdMolClass = 0;  // SHAKE kernel class: 0 <= 3 atoms/3 constraints, 1 <= 4/6, 2 <= 16/32
   // CUDA graph of mdGraphSteps whole steps (precision 1); rebuilt when stale
   int mdGraphSteps = 20, mdGraphK = 0;
-  long long mdGraphMainK = 0, mdGraphBodyK = 0;  // kernels per step / per rebuild
+  long long mdGraphMainK = 0, mdGraphBodyK = 0;  // kernels per launch / per rebuild
   long long mdGraphPruneK = 0;                   // kernels per prune
   double mdPruneBuf = 0.0;  // inner-list buffer (A) of the mixed form; 0 = no pruning
   mdbas::DBuf mdXp;         // positions at the last prune
@@ -105,8 +105,8 @@ struct mdbas_nb_engine {
   cudaGraphExec_t mdExec = nullptr;
   cudaStream_t mdCapStream = nullptr, mdSideStream = nullptr;
   // branches of the captured step (md.cu: MdBranch) and their fork/join events
-  cudaStream_t mdBranch[3] = {};
-  cudaEvent_t mdForkEv = nullptr, mdJoinEv[3] = {};
+  cudaStream_t mdBranch[4] = {};
+  cudaEvent_t mdForkEv = nullptr, mdJoinEv[4] = {};
   mdbas::DBuf mdRows, mdSnap;
 };
 

@@ -25,7 +25,8 @@ struct EwaldWork {
   double fact1 = 0.;  // 2 (2 pi / V) C of the last launch
 };
 
-constexpr int kSpmeEnergy = 6;  // SpmeWork::sums: 0-5 stress, 6 energy, 7-9 force sums
+// SpmeWork::sums: 0-5 stress, 6 energy, 7-9 force sums
+constexpr int kSpmeEnergy = 6, kSpmeForces = 7;
 struct SpmeWork {
   int device = -1;
   int m1 = 0, m2 = 0, m3 = 0, nbsp = 0, n = 0;

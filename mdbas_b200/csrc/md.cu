@@ -14,7 +14,13 @@
 //            src/shake.c:328-456), kinetic energy (kinetic, src/utils.c:502),
 //            positions wrapped into the box (image_update).
 // Everything stays on the GPU; the host only reads one word per step (the
-// displacement test) and the energies when asked.
+// displacement test) and the energies when asked, or nothing during the steps
+// of a captured run.  What a step does to each atom is in few kernels: stage 1
+// (the bath's scaling of the step before, kick, drift, constraints of rigid
+// triangles, displacement test, decision), stage 2 (the force parts summed,
+// kick, constraints) and the step's end (kinetic energy, wrapping).  As 14
+// kernels and six fills, with gaps of 1 to 2 us, they took 100 of the 441 us
+// of a step of 96,000 atoms of water.
 //
 // Constraints are solved molecule by molecule (connected components of the
 // constraint graph, one thread each) with MDBas's iteration: every constraint
@@ -44,34 +50,245 @@ constexpr int kMolTinyAtoms = 3, kMolTinyCons = 3;      // rigid water, X-H bond
 constexpr int kMolSmallAtoms = 4, kMolSmallCons = 6;    // CH3, NH3+ ...
 constexpr int kMolMaxAtoms = 16, kMolMaxCons = 32;      // the largest accepted
 
-// stage 1 of vv_nve: half kick then drift (src/integrate.c:1555-1580)
-// (atoms with skip[i] != 0 are integrated by the fused rigid-triangle kernels)
-__global__ void k_vv_stage1(int n, double dt, const double *__restrict__ fx,
-                            const double *__restrict__ fy, const double *__restrict__ fz,
-                            const double *__restrict__ rmass, double *__restrict__ vx,
-                            double *__restrict__ vy, double *__restrict__ vz,
-                            double *__restrict__ x, double *__restrict__ y,
-                            double *__restrict__ z, const int *__restrict__ skip) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || (skip && skip[i])) return;
-  vx[i] += 0.5 * dt * fx[i] * rmass[i];
-  vy[i] += 0.5 * dt * fy[i] * rmass[i];
-  vz[i] += 0.5 * dt * fz[i] * rmass[i];
-  x[i] += dt * vx[i];
-  y[i] += dt * vy[i];
-  z[i] += dt * vz[i];
+// Slots of the engine's MD word buffer (int64 each).
+enum MdWord {
+  W_DISP = 0,     // largest squared displacement since the last build (bits)
+  W_FLAGS = 1,    // OR of the fixed-point error bits of the recorded steps
+  W_KIN = 2,      // kinetic energy, fixed point (2^-24)
+  W_KIN2 = 9,     // the same of every second captured step
+  W_DISP2 = 3,    // largest squared displacement since the last prune (bits)
+  W_SHAKE = 4,    // two ints: SHAKE error bits, largest iteration count
+  W_DONE = 5,     // finished blocks of the displacement test
+  W_STEP = 6,     // device step counter (graph form)
+  W_BUILDS = 7,   // list builds inside the graph since the last read
+  W_PRUNES = 8,   // prunes inside the graph since the last read
+  W_COUNT = 10
+};
+
+// The record of a step: fixed-point energies {direct, correction, vdw,
+// kinetic, bonded, reciprocal} (2^-24); the step's error bits go to W_FLAGS.
+constexpr int kRowWords = 6;
+__global__ void k_md_row(long long *__restrict__ row, const long long *__restrict__ acc,
+                         const long long *__restrict__ kin, const long long *__restrict__ bonded,
+                         const long long *__restrict__ kspace, long long *__restrict__ word) {
+  if (threadIdx.x != 0) return;
+  row[0] = acc[ACC_E_DIR];
+  row[1] = acc[ACC_E_CORR];
+  row[2] = acc[ACC_E_VDW];
+  row[3] = kin[0];
+  row[4] = bonded ? bonded[0] : 0;
+  row[5] = kspace ? kspace[0] : 0;
+  atomicOr(reinterpret_cast<unsigned long long *>(word + W_FLAGS),
+           (unsigned long long)acc[ACC_FLAGS]);
 }
 
-__global__ void k_vv_kick(int n, double dt, const double *__restrict__ fx,
-                          const double *__restrict__ fy, const double *__restrict__ fz,
-                          const double *__restrict__ rmass, double *__restrict__ vx,
-                          double *__restrict__ vy, double *__restrict__ vz,
-                          const int *__restrict__ skip) {
+// What a captured step decides once its positions are known.
+struct MdDecide {
+  cudaGraphConditionalHandle hB, hP;
+  double half2, halfIn2;
+  int update, prune;
+  int kin;  // the step's kinetic-energy word (W_KIN or W_KIN2)
+};
+
+// One thread.  Set the rebuild condition (hB) from the largest squared
+// displacement since the build, or from MDBas's fixed cadence "list N" (step %
+// N == 0) when update > 0, and the prune condition (hP: a rebuild, or the
+// displacement since the last prune past halfIn2; never when prune = 0);
+// advance the device step counter; clear the words that the step adds to.
+__device__ void decide(const MdDecide &d, long long *word) {
+  const long long st = word[W_STEP] + 1;
+  word[W_STEP] = st;
+  const bool rebuild =
+      d.update > 0 ? (st % d.update) == 0 : __longlong_as_double(word[W_DISP]) > d.half2;
+  const bool pr = d.prune && (rebuild || __longlong_as_double(word[W_DISP2]) > d.halfIn2);
+  cudaGraphSetConditional(d.hB, rebuild ? 1u : 0u);
+  if (d.prune) cudaGraphSetConditional(d.hP, pr ? 1u : 0u);
+  word[W_DISP] = 0;
+  word[W_DISP2] = 0;
+  word[d.kin] = 0;
+}
+
+// The displacement test: largest squared displacement since the last build
+// (minimum image) and, when xp is given, since the last prune, into W_DISP and
+// W_DISP2 as the bit patterns of non-negative doubles (which order like the
+// doubles); the block that finishes last decides (active).
+struct MdDisp {
+  const double *xb, *yb, *zb, *xp, *yp, *zp;  // xb null: no test
+  long long *word;
+  int active;
+  MdDecide d;
+};
+
+__device__ __forceinline__ void disp_atom(const MdDisp &m, const DevBox &b, int i, double x,
+                                          double y, double z, double &r2, double &p2) {
+  double dx = x - m.xb[i], dy = y - m.yb[i], dz = z - m.zb[i];
+  const double r = dist_d(b, dx, dy, dz);
+  r2 = r == r ? fmax(r2, r) : 1e300;  // NaN forces a rebuild (which reports it)
+  if (m.xp) {
+    double ex = x - m.xp[i], ey = y - m.yp[i], ez = z - m.zp[i];
+    const double p = dist_d(b, ex, ey, ez);
+    p2 = p == p ? fmax(p2, p) : 1e300;
+  }
+}
+
+// Every thread of the block.
+__device__ __forceinline__ void disp_finish(const MdDisp &m, double r2, double p2) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+    p2 = fmax(p2, __shfl_xor_sync(0xffffffffu, p2, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    unsigned long long *w = reinterpret_cast<unsigned long long *>(m.word);
+    atomicMax(w + W_DISP, (unsigned long long)__double_as_longlong(r2));
+    if (m.xp) atomicMax(w + W_DISP2, (unsigned long long)__double_as_longlong(p2));
+    __threadfence();
+  }
+  if (!m.active) return;
+  __syncthreads();
+  if (threadIdx.x == 0 &&
+      atomicInc(reinterpret_cast<unsigned *>(m.word + W_DONE), gridDim.x - 1) == gridDim.x - 1) {
+    __threadfence();
+    decide(m.d, m.word);
+  }
+}
+
+// Berendsen scaling of vv_nvt_b (src/integrate.c:1722-1733): lambda from the
+// kinetic energy summed on the device.  Inside a captured run a step's scaling
+// is made by the next step's first kernel as it reads the velocities.
+struct MdScale {
+  const long long *kin;  // null: none
+  double dtOverTau, kinTemp0;
+};
+
+__device__ __forceinline__ double scale_of(const MdScale &s) {
+  if (!s.kin) return 1.;
+  const double kin = (double)(*s.kin) / kEnergyScale;
+  return kin > 0. ? sqrt(1.0 + s.dtOverTau * (s.kinTemp0 / kin - 1.0)) : 1.;
+}
+
+// How a step's forces come together (energy(), src/energy.c:167-201): the
+// nonbonded ones from fixed point and slot order, the reciprocal ones minus
+// their mean (src/spme.c:684-697), the bonded terms in slot order, zero for
+// frozen atoms (freeze_atoms).  Null members are left out; without facc the
+// sum starts from f.
+struct ForceSum {
+  double *f;  // 3n, caller order
+  int n;
+  const int *slotOf;
+  const long long *facc;
+  int fstride;
+  const double *fr, *fsum;
+  const int *bStart, *bSlot;
+  const double *contrib;
+  int nSlots;
+  const int *frozen;
+};
+
+// Atom i's force into f and (fx, fy, fz); false for a frozen atom.
+__device__ __forceinline__ bool sum_forces(const ForceSum &s, int i, double &fx, double &fy,
+                                           double &fz) {
+  const size_t n = s.n;
+  if (s.facc) {
+    const int k = s.slotOf[i];
+    const double inv = 1.0 / kForceScale;
+    fx = (double)s.facc[k] * inv;
+    fy = (double)s.facc[(size_t)s.fstride + k] * inv;
+    fz = (double)s.facc[2 * (size_t)s.fstride + k] * inv;
+  } else {
+    fx = s.f[i];
+    fy = s.f[n + i];
+    fz = s.f[2 * n + i];
+  }
+  if (s.fr) {
+    const double inv = 1.0 / (double)s.n;
+    fx += s.fr[i] - s.fsum[0] * inv;
+    fy += s.fr[n + i] - s.fsum[1] * inv;
+    fz += s.fr[2 * n + i] - s.fsum[2] * inv;
+  }
+  if (s.bStart)
+    for (int k = s.bStart[i], end = s.bStart[i + 1]; k < end; ++k) {
+      const int slot = s.bSlot[k];
+      fx += s.contrib[slot];
+      fy += s.contrib[s.nSlots + slot];
+      fz += s.contrib[2 * (size_t)s.nSlots + slot];
+    }
+  const bool free = !(s.frozen && s.frozen[i]);
+  if (!free) fx = fy = fz = 0.;
+  s.f[i] = fx;
+  s.f[n + i] = fy;
+  s.f[2 * n + i] = fz;
+  return free;
+}
+
+// kinetic energy (src/utils.c:502-515), sum in fixed point (2^-24 units).
+// A term at or above termLimit (2^62 / n in fixed-point units, so that no
+// sum of n terms can wrap) or not finite raises FLAG_OVERFLOW in W_FLAGS.
+struct MdKin {
+  const double *mass;  // null: not wanted
+  double termLimit;
+  long long *sum, *word;
+};
+
+__device__ __forceinline__ long long kin_term(const MdKin &k, double mass, double vx, double vy,
+                                              double vz) {
+  const double t = 0.5 * mass * (vx * vx + vy * vy + vz * vz);
+  if (t * kEnergyScale < k.termLimit) return fix_e(t);
+  atomicOr(reinterpret_cast<unsigned long long *>(k.word + W_FLAGS),
+           (unsigned long long)FLAG_OVERFLOW);
+  return 0;
+}
+
+// Every lane of the warp.
+__device__ __forceinline__ void kin_finish(const MdKin &k, long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red_add(k.sum, v);
+}
+
+// stage 1 of vv_nve: half kick then drift (src/integrate.c:1555-1580)
+// (atoms with skip[i] != 0 are integrated by the fused rigid-triangle
+// kernels), and the displacement test where no constraints follow
+__global__ void __launch_bounds__(256)
+k_vv_stage1(int n, const DevBox *__restrict__ boxes, const int *__restrict__ atomRep, double dt,
+            const double *__restrict__ fx, const double *__restrict__ fy,
+            const double *__restrict__ fz, const double *__restrict__ rmass,
+            double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz,
+            double *__restrict__ x, double *__restrict__ y, double *__restrict__ z,
+            const int *__restrict__ skip, MdScale sc, MdDisp disp) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double r2 = 0., p2 = 0.;
+  if (i < n && !(skip && skip[i])) {
+    const double lam = scale_of(sc);
+    const double rm = rmass[i];
+    const double ux = dmul(vx[i], lam) + 0.5 * dt * fx[i] * rm;
+    const double uy = dmul(vy[i], lam) + 0.5 * dt * fy[i] * rm;
+    const double uz = dmul(vz[i], lam) + 0.5 * dt * fz[i] * rm;
+    const double px = x[i] + dt * ux, py = y[i] + dt * uy, pz = z[i] + dt * uz;
+    vx[i] = ux;
+    vy[i] = uy;
+    vz[i] = uz;
+    x[i] = px;
+    y[i] = py;
+    z[i] = pz;
+    if (disp.xb) disp_atom(disp, boxes[atomRep ? atomRep[i] : 0], i, px, py, pz, r2, p2);
+  }
+  if (disp.xb) disp_finish(disp, r2, p2);
+}
+
+// stage 2: the step's forces and the half kick
+__global__ void __launch_bounds__(256)
+k_vv_stage2(int n, double dt, ForceSum fs, const double *__restrict__ rmass,
+            double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz,
+            const int *__restrict__ skip) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || (skip && skip[i])) return;
-  vx[i] += 0.5 * dt * fx[i] * rmass[i];
-  vy[i] += 0.5 * dt * fy[i] * rmass[i];
-  vz[i] += 0.5 * dt * fz[i] * rmass[i];
+  double fx, fy, fz;
+  const bool free = sum_forces(fs, i, fx, fy, fz);
+  const double rm = rmass[i];
+  vx[i] = (free ? vx[i] : 0.) + 0.5 * dt * fx * rm;
+  vy[i] = (free ? vy[i] : 0.) + 0.5 * dt * fy * rm;
+  vz[i] = (free ? vz[i] : 0.) + 0.5 * dt * fz * rm;
 }
 
 // constraint vectors before the drift, minimum image (dist2, src/utils.c:82)
@@ -459,11 +676,13 @@ k_tri_stage1(int nTri, const DevBox *__restrict__ boxes, const int *__restrict__
              const double *__restrict__ fz, const double *__restrict__ rmass,
              double *__restrict__ x, double *__restrict__ y, double *__restrict__ z,
              double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz,
-             int *__restrict__ status) {
+             int *__restrict__ status, MdScale sc, MdDisp disp) {
   constexpr int LA[3] = {0, 0, 1}, LB[3] = {1, 2, 2};
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   int icycle = 0;
+  double r2 = 0., p2 = 0.;
   if (m < nTri) {
+    const double lam = scale_of(sc);
     const int4 t = tri[m];
     const int A[3] = {t.x, t.y, t.z};
     const DevBox &b = boxes[atomRep ? atomRep[t.x] : 0];
@@ -478,9 +697,9 @@ k_tri_stage1(int nTri, const DevBox *__restrict__ boxes, const int *__restrict__
       px[i] = x[A[i]];
       py[i] = y[A[i]];
       pz[i] = z[A[i]];
-      qx[i] = vx[A[i]];
-      qy[i] = vy[A[i]];
-      qz[i] = vz[A[i]];
+      qx[i] = dmul(vx[A[i]], lam);
+      qy[i] = dmul(vy[A[i]], lam);
+      qz[i] = dmul(vz[A[i]], lam);
       rm[i] = rmass[A[i]];
     }
     // constraint vectors before the drift
@@ -565,20 +784,20 @@ k_tri_stage1(int nTri, const DevBox *__restrict__ boxes, const int *__restrict__
       vx[A[i]] = qx[i];
       vy[A[i]] = qy[i];
       vz[A[i]] = qz[i];
+      if (disp.xb) disp_atom(disp, b, A[i], px[i], py[i], pz[i], r2, p2);
     }
   }
   report_cycles(status, icycle);
+  if (disp.xb) disp_finish(disp, r2, p2);
 }
 
 __global__ void __launch_bounds__(128)
 k_tri_stage2(int nTri, const DevBox *__restrict__ boxes, const int *__restrict__ atomRep,
              double dt, double tolvel, int maxCycle,
-             const int4 *__restrict__ tri, const double *__restrict__ fx,
-             const double *__restrict__ fy, const double *__restrict__ fz,
-             const double *__restrict__ rmass, const double *__restrict__ x,
-             const double *__restrict__ y, const double *__restrict__ z,
-             double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz,
-             int *__restrict__ status) {
+             const int4 *__restrict__ tri, ForceSum fs, const double *__restrict__ rmass,
+             const double *__restrict__ x, const double *__restrict__ y,
+             const double *__restrict__ z, double *__restrict__ vx, double *__restrict__ vy,
+             double *__restrict__ vz, int *__restrict__ status) {
   constexpr int LA[3] = {0, 0, 1}, LB[3] = {1, 2, 2};
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= nTri) return;
@@ -592,9 +811,11 @@ k_tri_stage2(int nTri, const DevBox *__restrict__ boxes, const int *__restrict__
     py[i] = y[A[i]];
     pz[i] = z[A[i]];
     rm[i] = rmass[A[i]];
-    qx[i] = vx[A[i]] + 0.5 * dt * fx[A[i]] * rm[i];
-    qy[i] = vy[A[i]] + 0.5 * dt * fy[A[i]] * rm[i];
-    qz[i] = vz[A[i]] + 0.5 * dt * fz[A[i]] * rm[i];
+    double fx, fy, fz;
+    const bool free = sum_forces(fs, A[i], fx, fy, fz);
+    qx[i] = (free ? vx[A[i]] : 0.) + 0.5 * dt * fx * rm[i];
+    qy[i] = (free ? vy[A[i]] : 0.) + 0.5 * dt * fy * rm[i];
+    qz[i] = (free ? vz[A[i]] : 0.) + 0.5 * dt * fz * rm[i];
   }
   // constraint vectors at the new positions; the denominators are fixed
   double dcx[3], dcy[3], dcz[3], dd2[3], trm[3][2], iden[3];
@@ -649,139 +870,73 @@ k_tri_stage2(int nTri, const DevBox *__restrict__ boxes, const int *__restrict__
   }
 }
 
-// positions back into their box (image_update, src/utils.c:162-218)
-__global__ void k_wrap(int n, const DevBox *__restrict__ boxes, const int *__restrict__ atomRep,
-                       double *__restrict__ x, double *__restrict__ y, double *__restrict__ z) {
+// The end of a step: kinetic energy, and positions back into their box
+// (image_update, src/utils.c:162-218)
+__global__ void __launch_bounds__(256)
+k_kin_wrap(int n, const DevBox *__restrict__ boxes, const int *__restrict__ atomRep,
+           double *__restrict__ x, double *__restrict__ y, double *__restrict__ z,
+           const double *__restrict__ vx, const double *__restrict__ vy,
+           const double *__restrict__ vz, MdKin kin) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double xi = x[i], yi = y[i], zi = z[i];
-  image_d(boxes[atomRep ? atomRep[i] : 0], xi, yi, zi);
-  x[i] = xi;
-  y[i] = yi;
-  z[i] = zi;
-}
-
-// kinetic energy (src/utils.c:502-515), sum in fixed point (2^-24 units).
-// A term at or above termLimit (2^62 / n in fixed-point units, so that no
-// sum of n terms can wrap) or not finite raises FLAG_OVERFLOW in *flags.
-__global__ void k_kinetic(int n, const double *__restrict__ mass, const double *__restrict__ vx,
-                          const double *__restrict__ vy, const double *__restrict__ vz,
-                          double termLimit, long long *__restrict__ acc,
-                          long long *__restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  long long v = 0;
+  long long term = 0;
   if (i < n) {
-    const double t = 0.5 * mass[i] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
-    if (!(t * kEnergyScale < termLimit)) {
-      atomicOr(reinterpret_cast<unsigned long long *>(flags), (unsigned long long)FLAG_OVERFLOW);
-    } else {
-      v = fix_e(t);
-    }
+    if (kin.mass) term = kin_term(kin, kin.mass[i], vx[i], vy[i], vz[i]);
+    double xi = x[i], yi = y[i], zi = z[i];
+    image_d(boxes[atomRep ? atomRep[i] : 0], xi, yi, zi);
+    x[i] = xi;
+    y[i] = yi;
+    z[i] = zi;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red_add(acc, v);
+  if (kin.mass) kin_finish(kin, term);
 }
 
-// largest squared displacement since the last build (minimum image) and,
-// when xp is given, since the last prune; each as the bit pattern of a
-// non-negative double (which orders like the double)
-__global__ void k_max_disp(int n, const DevBox *__restrict__ boxes,
-                           const int *__restrict__ atomRep, const double *__restrict__ x,
-                           const double *__restrict__ y, const double *__restrict__ z,
-                           const double *__restrict__ xb, const double *__restrict__ yb,
-                           const double *__restrict__ zb, const double *__restrict__ xp,
-                           const double *__restrict__ yp, const double *__restrict__ zp,
-                           unsigned long long *__restrict__ outB,
-                           unsigned long long *__restrict__ outP) {
+// The displacement test alone, after constraint kernels.
+__global__ void __launch_bounds__(256)
+k_max_disp(int n, const DevBox *__restrict__ boxes, const int *__restrict__ atomRep,
+           const double *__restrict__ x, const double *__restrict__ y,
+           const double *__restrict__ z, MdDisp disp) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double r2 = 0., p2 = 0.;
-  if (i < n) {
-    const DevBox &b = boxes[atomRep ? atomRep[i] : 0];
-    double dx = x[i] - xb[i], dy = y[i] - yb[i], dz = z[i] - zb[i];
-    r2 = dist_d(b, dx, dy, dz);
-    if (!(r2 == r2)) r2 = 1e300;  // NaN forces a rebuild (which reports it)
-    if (xp) {
-      double ex = x[i] - xp[i], ey = y[i] - yp[i], ez = z[i] - zp[i];
-      p2 = dist_d(b, ex, ey, ez);
-      if (!(p2 == p2)) p2 = 1e300;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
-    p2 = fmax(p2, __shfl_xor_sync(0xffffffffu, p2, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(outB, (unsigned long long)__double_as_longlong(r2));
-    if (xp) atomicMax(outP, (unsigned long long)__double_as_longlong(p2));
-  }
+  if (i < n) disp_atom(disp, boxes[atomRep ? atomRep[i] : 0], i, x[i], y[i], z[i], r2, p2);
+  disp_finish(disp, r2, p2);
 }
 
-// frozen atoms keep zero force and velocity (freeze_atoms, src/utils.c:131-150)
-__global__ void k_freeze(int n, const int *__restrict__ frozen, double *__restrict__ f,
-                         double *__restrict__ v) {
+// The forces alone; frozen atoms also get zero velocity (freeze_atoms,
+// src/utils.c:131-150).
+__global__ void k_sum_forces(ForceSum fs, double *__restrict__ v) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !frozen[i]) return;
-  f[i] = f[n + i] = f[2 * (size_t)n + i] = 0.;
-  v[i] = v[n + i] = v[2 * (size_t)n + i] = 0.;
+  if (i >= fs.n) return;
+  double fx, fy, fz;
+  if (!sum_forces(fs, i, fx, fy, fz)) v[i] = v[fs.n + i] = v[2 * (size_t)fs.n + i] = 0.;
 }
 
-// Berendsen scaling of vv_nvt_b (src/integrate.c:1722-1733): every thread
-// derives lambda from the kinetic energy summed on the device.
-__global__ void k_berendsen(int n, double dtOverTau, double kinTemp0,
-                            const long long *__restrict__ kfix, double *__restrict__ vx,
-                            double *__restrict__ vy, double *__restrict__ vz) {
+__global__ void k_berendsen(int n, MdScale sc, double *__restrict__ vx, double *__restrict__ vy,
+                            double *__restrict__ vz) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double kin = (double)(*kfix) / kEnergyScale;
-  if (!(kin > 0.)) return;
-  const double lambda = sqrt(1.0 + dtOverTau * (kinTemp0 / kin - 1.0));
+  const double lambda = scale_of(sc);
   vx[i] *= lambda;
   vy[i] *= lambda;
   vz[i] *= lambda;
 }
 
-// --- graph-only kernels: the rebuild decision and the per-step record -----
-// Set the rebuild condition (hB) from the largest squared displacement since
-// the build, or from MDBas's fixed cadence "list N" (step % N == 0) when
-// update > 0, and the prune condition (hP: a rebuild, or the displacement
-// since the last prune past halfIn2; never when prune = 0); advance the
-// device step counter.
-__global__ void k_decide(cudaGraphConditionalHandle hB, cudaGraphConditionalHandle hP,
-                         const unsigned long long *__restrict__ bitsB,
-                         const unsigned long long *__restrict__ bitsP, double half2,
-                         double halfIn2, int update, int prune,
-                         long long *__restrict__ stepDev) {
-  if (threadIdx.x != 0) return;
-  const long long st = stepDev[0] + 1;
-  stepDev[0] = st;
-  const bool rebuild = update > 0 ? (st % update) == 0
-                                  : __longlong_as_double((long long)bitsB[0]) > half2;
-  const bool pr = prune && (rebuild || __longlong_as_double((long long)bitsP[0]) > halfIn2);
-  cudaGraphSetConditional(hB, rebuild ? 1u : 0u);
-  if (prune) cudaGraphSetConditional(hP, pr ? 1u : 0u);
+// The decision without a displacement test (fixed cadence, no pruning).
+__global__ void k_decide(MdDecide d, long long *__restrict__ word) {
+  if (threadIdx.x == 0) decide(d, word);
+}
+
+__global__ void k_save_positions(int n, const double *__restrict__ x,
+                                 const double *__restrict__ y, const double *__restrict__ z,
+                                 double *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = x[i];
+  out[n + i] = y[i];
+  out[2 * (size_t)n + i] = z[i];
 }
 
 __global__ void k_count(long long *__restrict__ c) {
   if (threadIdx.x == 0) c[0] += 1;
-}
-
-// Fixed-point energies of the step (elec direct, elec corr, vdw, kinetic) and
-// the accumulated error bits.
-// row = {direct, correction, vdw, kinetic, bonded, reciprocal} in fixed
-// point (2^-24)
-__global__ void k_md_row(long long *__restrict__ row, const long long *__restrict__ acc,
-                         const long long *__restrict__ kin, const long long *__restrict__ bonded,
-                         const long long *__restrict__ kspace, long long *__restrict__ flags) {
-  if (threadIdx.x != 0) return;
-  row[0] = acc[ACC_E_DIR];
-  row[1] = acc[ACC_E_CORR];
-  row[2] = acc[ACC_E_VDW];
-  row[3] = kin[0];
-  row[4] = bonded ? bonded[0] : 0;
-  row[5] = kspace ? kspace[0] : 0;
-  flags[0] |= acc[ACC_FLAGS];
 }
 
 }  // namespace
@@ -801,21 +956,6 @@ __global__ void k_md_row(long long *__restrict__ row, const long long *__restric
 
 namespace {
 
-// Slots of the engine's MD word buffer (int64 each).
-enum MdWord {
-  W_DISP = 0,     // largest squared displacement since the last build (bits)
-  W_FLAGS = 1,    // OR of the fixed-point error bits of the recorded steps
-  W_KIN = 2,      // kinetic energy, fixed point (2^-24)
-  W_SHAKE = 4,    // two ints: SHAKE error bits, largest iteration count
-  W_STEP = 6,     // device step counter (graph form)
-  W_BUILDS = 7,   // list builds inside the graph since the last read
-  W_DISP2 = 3,    // largest squared displacement since the last prune (bits)
-  W_PRUNES = 8,   // prunes inside the graph since the last read
-  W_COUNT = 10
-};
-
-constexpr int kRowWords = 6;  // k_md_row's row length
-
 // Fixed-point bonded energy of the last md_forces (null without bonded terms).
 const long long *md_bonded_fix(const mdbas_nb_engine *e) {
   return e->bonded.nTerms() > 0 ? e->bonded.sums.as<long long>() + BS_FIX : nullptr;
@@ -833,40 +973,60 @@ int md_bonded_terms(mdbas_nb_engine *e, cudaStream_t s) {
                       e->z.as<double>(), s);
 }
 
-// FP64 forces of the last compute, caller order, into e->mdF (3n); then the
-// reciprocal forces and bonded terms (of md_kspace_terms and md_bonded_terms)
-// in MDBas's order (energy(), src/energy.c:167-190) and the frozen atoms
-// (freeze_atoms, src/energy.c:198-201).
-int md_sum_forces(mdbas_nb_engine *e, cudaStream_t s) {
+// The parts of the last evaluation's forces (with md_kspace_terms and
+// md_bonded_terms) that the second half kick adds up into e->mdF (3n, caller
+// order).  Explicit Ewald forces are added here: they have a kernel of their
+// own.
+int md_force_parts(mdbas_nb_engine *e, ForceSum &fs, cudaStream_t s) {
   const int n = e->n;
   double *f = e->mdF.as<double>();
+  fs = ForceSum{};
+  fs.f = f;
+  fs.n = n;
   if (e->cfg.precision == 0) {
     MDB_CUDA(cudaMemcpyAsync(f, e->f64.p, sizeof(double) * 3 * (size_t)n,
                              cudaMemcpyDeviceToDevice, s));
-  } else {
+  } else if (e->kspaceKind == 1) {
     MDB_TRY(forces_out_launch(e->cl, n, 0, f, f + n, f + 2 * (size_t)n, s));
+  } else {
+    fs.slotOf = e->cl.slotOf.as<int>();
+    fs.facc = e->cl.facc.as<long long>();
+    fs.fstride = e->cl.slotCap;
   }
-  MDB_TRY(md_kspace_add(e, f, s));
-  MDB_TRY(bonded_add(e->bonded, f, s));
-  if (e->hasFrozen)
-    MDB_LAUNCH(k_freeze, grid_for(n, 256), 256, 0, s, n, e->frozen.as<int>(), f,
-               e->mdV.as<double>());
+  if (e->kspaceKind == 1) MDB_TRY(md_kspace_add(e, f, s));
+  if (e->kspaceKind == 2) {
+    fs.fr = e->kSpme->fr.as<double>();
+    fs.fsum = e->kSpme->sums.as<double>() + kSpmeForces;
+  }
+  if (e->bonded.nTerms() > 0) {
+    fs.bStart = e->bonded.atomStart.as<int>();
+    fs.bSlot = e->bonded.atomSlot.as<int>();
+    fs.contrib = e->bonded.contrib.as<double>();
+    fs.nSlots = e->bonded.nSlots();
+  }
+  if (e->hasFrozen) fs.frozen = e->frozen.as<int>();
   return MDBAS_NB_OK;
 }
 
+// The whole sum into e->mdF, for the first step.
 int md_forces(mdbas_nb_engine *e, cudaStream_t s) {
+  const int n = e->n;
   MDB_TRY(md_kspace_terms(e, s));
   MDB_TRY(md_bonded_terms(e, s));
-  return md_sum_forces(e, s);
+  ForceSum fs;
+  MDB_TRY(md_force_parts(e, fs, s));
+  MDB_LAUNCH(k_sum_forces, grid_for(n, 256), 256, 0, s, fs, e->mdV.as<double>());
+  return MDBAS_NB_OK;
+}
+
+int md_save_positions(mdbas_nb_engine *e, double *out, cudaStream_t s) {
+  MDB_LAUNCH(k_save_positions, grid_for(e->n, 256), 256, 0, s, e->n, e->x.as<double>(),
+             e->y.as<double>(), e->z.as<double>(), out);
+  return MDBAS_NB_OK;
 }
 
 int md_save_build_positions(mdbas_nb_engine *e, cudaStream_t s) {
-  const size_t bytes = sizeof(double) * (size_t)e->n;
-  double *xb = e->mdXb.as<double>();
-  MDB_CUDA(cudaMemcpyAsync(xb, e->x.p, bytes, cudaMemcpyDeviceToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(xb + e->n, e->y.p, bytes, cudaMemcpyDeviceToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(xb + 2 * (size_t)e->n, e->z.p, bytes, cudaMemcpyDeviceToDevice, s));
-  return MDBAS_NB_OK;
+  return md_save_positions(e, e->mdXb.as<double>(), s);
 }
 
 // Synchronising list build (either precision) at the current positions.
@@ -878,30 +1038,66 @@ int md_build(mdbas_nb_engine *e) {
   return MDBAS_NB_OK;
 }
 
-// stage 1 of vv_nve: constraint vectors, half kick + drift, SHAKE on positions
-int md_stage1(mdbas_nb_engine *e, cudaStream_t s) {
+bool md_prune_on(const mdbas_nb_engine *e) {
+  return e->cfg.precision == 1 && e->mdPruneBuf > 0.;
+}
+
+// The displacement test of a step (none with a fixed cadence and no pruning).
+MdDisp md_disp(const mdbas_nb_engine *e) {
+  MdDisp m{};
+  if (e->mdListUpdate > 0 && !md_prune_on(e)) return m;
+  const size_t n = e->n;
+  m.xb = e->mdXb.as<double>();
+  m.yb = m.xb + n;
+  m.zb = m.yb + n;
+  m.word = e->mdWord.as<long long>();
+  if (!md_prune_on(e)) return m;
+  m.xp = e->mdXp.as<double>();
+  m.yp = m.xp + n;
+  m.zp = m.yp + n;
+  return m;
+}
+
+int md_max_disp(mdbas_nb_engine *e, cudaStream_t s, const MdDisp &disp) {
+  if (disp.xb)
+    MDB_LAUNCH(k_max_disp, grid_for(e->n, 256), 256, 0, s, e->n, BOXES(e), e->x.as<double>(),
+               e->y.as<double>(), e->z.as<double>(), disp);
+  return MDBAS_NB_OK;
+}
+
+// One kernel moves all atoms in stage 1, and can test the displacements:
+// unconstrained systems, or all atoms in rigid triangles.
+bool md_one_kernel(const mdbas_nb_engine *e) {
+  return e->mdTri ? e->mdNTri == e->n : e->mdNCons == 0;
+}
+
+// stage 1 of vv_nve: constraint vectors, half kick + drift, SHAKE on
+// positions; then the displacement test, if disp has one
+int md_stage1(mdbas_nb_engine *e, cudaStream_t s, const MdScale &sc, const MdDisp &disp) {
   const int n = e->n, nc = e->mdNCons;
   double *x = e->x.as<double>(), *y = e->y.as<double>(), *z = e->z.as<double>();
   double *vx = e->mdV.as<double>(), *vy = vx + n, *vz = vy + n;
   const double *fx = e->mdF.as<double>(), *fy = fx + n, *fz = fy + n;
   double *ddx = e->mdDd.as<double>(), *ddy = ddx + nc, *ddz = ddy + nc;
+  const MdDisp none{};
+  const MdDisp &first = md_one_kernel(e) ? disp : none;
   if (e->mdTri) {
     // rigid triangles: vectors, kick, drift and SHAKE fused per molecule;
     // the atom kernel integrates the unconstrained atoms only
     if (e->mdNTri < n)
-      MDB_LAUNCH(k_vv_stage1, grid_for(n, 256), 256, 0, s, n, e->mdDt, fx, fy, fz,
-                 e->mdRmass.as<double>(), vx, vy, vz, x, y, z, e->mdNAt.as<int>());
+      MDB_LAUNCH(k_vv_stage1, grid_for(n, 256), 256, 0, s, n, BOXES(e), e->mdDt, fx, fy, fz,
+                 e->mdRmass.as<double>(), vx, vy, vz, x, y, z, e->mdNAt.as<int>(), sc, none);
     MDB_LAUNCH(k_tri_stage1, grid_for(e->mdNMol, 128), 128, 0, s, e->mdNMol, BOXES(e), e->mdDt,
                e->mdTol, e->mdMaxCycle, e->mdTriAtoms.as<int4>(), e->mdTriLen2.as<double4>(),
                fx, fy, fz, e->mdRmass.as<double>(), x, y, z, vx, vy, vz,
-               reinterpret_cast<int *>(e->mdWord.as<long long>() + W_SHAKE));
-    return MDBAS_NB_OK;
+               reinterpret_cast<int *>(e->mdWord.as<long long>() + W_SHAKE), sc, first);
+    return md_max_disp(e, s, first.xb ? none : disp);
   }
   if (nc > 0)
     MDB_LAUNCH(k_cons_vectors, grid_for(nc, 256), 256, 0, s, nc, BOXES(e), e->mdCa.as<int>(),
                e->mdCb.as<int>(), x, y, z, ddx, ddy, ddz);
-  MDB_LAUNCH(k_vv_stage1, grid_for(n, 256), 256, 0, s, n, e->mdDt, fx, fy, fz,
-             e->mdRmass.as<double>(), vx, vy, vz, x, y, z, nullptr);
+  MDB_LAUNCH(k_vv_stage1, grid_for(n, 256), 256, 0, s, n, BOXES(e), e->mdDt, fx, fy, fz,
+             e->mdRmass.as<double>(), vx, vy, vz, x, y, z, nullptr, sc, first);
   if (nc > 0) {
     auto shake = e->mdMolClass == 0   ? k_shake_positions<kMolTinyAtoms, kMolTinyCons>
                  : e->mdMolClass == 1 ? k_shake_positions<kMolSmallAtoms, kMolSmallCons>
@@ -912,26 +1108,7 @@ int md_stage1(mdbas_nb_engine *e, cudaStream_t s) {
                e->mdNAt.as<int>(), x, y, z, vx, vy, vz,
                reinterpret_cast<int *>(e->mdWord.as<long long>() + W_SHAKE));
   }
-  return MDBAS_NB_OK;
-}
-
-bool md_prune_on(const mdbas_nb_engine *e) {
-  return e->cfg.precision == 1 && e->mdPruneBuf > 0.;
-}
-
-int md_max_disp(mdbas_nb_engine *e, cudaStream_t s) {
-  const int n = e->n;
-  long long *word = e->mdWord.as<long long>();
-  const double *xb = e->mdXb.as<double>();
-  const double *xp = md_prune_on(e) ? e->mdXp.as<double>() : nullptr;
-  MDB_CUDA(cudaMemsetAsync(word + W_DISP, 0, sizeof(long long), s));
-  MDB_CUDA(cudaMemsetAsync(word + W_DISP2, 0, sizeof(long long), s));
-  MDB_LAUNCH(k_max_disp, grid_for(n, 256), 256, 0, s, n, BOXES(e), e->x.as<double>(),
-             e->y.as<double>(), e->z.as<double>(), xb, xb + n, xb + 2 * (size_t)n, xp,
-             xp ? xp + n : nullptr, xp ? xp + 2 * (size_t)n : nullptr,
-             reinterpret_cast<unsigned long long *>(word + W_DISP),
-             reinterpret_cast<unsigned long long *>(word + W_DISP2));
-  return MDBAS_NB_OK;
+  return md_max_disp(e, s, first.xb ? none : disp);
 }
 
 // Inner radius of the pruned list: the cut-off plus the prune buffer, with the
@@ -944,12 +1121,7 @@ float md_rin2(const mdbas_nb_engine *e) {
 // Prune the list at the current (refreshed) layout and save the positions.
 int md_prune(mdbas_nb_engine *e, cudaStream_t s) {
   MDB_TRY(cluster_prune(e->cl, md_rin2(e), s));
-  const size_t bytes = sizeof(double) * (size_t)e->n;
-  double *xp = e->mdXp.as<double>();
-  MDB_CUDA(cudaMemcpyAsync(xp, e->x.p, bytes, cudaMemcpyDeviceToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(xp + e->n, e->y.p, bytes, cudaMemcpyDeviceToDevice, s));
-  MDB_CUDA(cudaMemcpyAsync(xp + 2 * (size_t)e->n, e->z.p, bytes, cudaMemcpyDeviceToDevice, s));
-  return MDBAS_NB_OK;
+  return md_save_positions(e, e->mdXp.as<double>(), s);
 }
 
 // Host-driven prune (outside graphs): also switches the pair kernel over.
@@ -966,7 +1138,10 @@ int md_prune_sync(mdbas_nb_engine *e) {
 // pair kernel of 10,000 atoms leaves most of the chip idle for its 52 us, and
 // the 16 kernels of its SPME take 105: a step of flexible chains with SPME
 // 196 -> 160 us; of 96,000 atoms of water (the exclusions' 11 us) 441 -> 434.
-enum MdBranch { BR_KSPACE = 0, BR_BONDED = 1, BR_EXCL = 2 };
+// With the small kernels folded into the half kicks besides, 149 and 399.
+// BR_SIDE takes what leaves the step's own path free: the record of a step
+// (during the next one's stage 1) and the clearing of the force words.
+enum MdBranch { BR_KSPACE = 0, BR_BONDED = 1, BR_EXCL = 2, BR_SIDE = 3 };
 
 int md_fork(mdbas_nb_engine *e, MdBranch b, cudaStream_t s) {
   MDB_CUDA(cudaEventRecord(e->mdForkEv, s));
@@ -990,16 +1165,16 @@ int md_fork_terms(mdbas_nb_engine *e, cudaStream_t s) {
     MDB_TRY(md_fork(e, BR_BONDED, s));
     MDB_TRY(md_bonded_terms(e, e->mdBranch[BR_BONDED]));
   }
-  return MDBAS_NB_OK;
+  MDB_TRY(md_fork(e, BR_SIDE, s));
+  return cluster_clear(e->cl, e->mdBranch[BR_SIDE]);
 }
 
 // Forces of a captured step on the current layout (refreshed by the caller):
-// evaluate, join the branches, convert to caller order.
+// evaluate, join the branches.
 int md_forces_cluster(mdbas_nb_engine *e, cudaStream_t s) {
   ClusterWork &w = e->cl;
   const int n = e->n;
-  MDB_CUDA(cudaMemsetAsync(w.facc.p, 0, sizeof(long long) * 3 * (size_t)w.slotCap, s));
-  MDB_CUDA(cudaMemsetAsync(w.acc.p, 0, sizeof(long long) * ACC_COUNT, s));
+  MDB_TRY(md_join(e, BR_SIDE, s));  // facc and acc are clear
   MDB_TRY(md_fork(e, BR_EXCL, s));
   MDB_TRY(excl_fix_launch(w, n, e->pp, e->exclStartSym.as<int>(), e->exclFlatSym.as<int>(),
                           e->x.as<double>(), e->y.as<double>(), e->z.as<double>(),
@@ -1008,7 +1183,7 @@ int md_forces_cluster(mdbas_nb_engine *e, cudaStream_t s) {
   MDB_TRY(md_join(e, BR_EXCL, s));
   if (e->kspaceKind != 0) MDB_TRY(md_join(e, BR_KSPACE, s));
   if (e->bonded.nTerms() > 0) MDB_TRY(md_join(e, BR_BONDED, s));
-  return md_sum_forces(e, s);
+  return MDBAS_NB_OK;
 }
 
 int md_refresh_cluster(mdbas_nb_engine *e, cudaStream_t s) {
@@ -1016,29 +1191,31 @@ int md_refresh_cluster(mdbas_nb_engine *e, cudaStream_t s) {
                          e->q.as<double>(), sqrt(e->cfg.chargeConst), s);
 }
 
-// stage 2: half kick, RATTLE on velocities, kinetic energy (+ Berendsen),
-// positions wrapped into the box
-int md_stage2(mdbas_nb_engine *e, cudaStream_t s, bool kin, double tauT, double kinTemp0) {
+// stage 2: the forces summed, half kick, RATTLE on velocities, kinetic energy
+// (into the given word, cleared by the caller; -1: not wanted), positions
+// wrapped into the box (image_update, src/integrate.c:1626)
+int md_stage2(mdbas_nb_engine *e, cudaStream_t s, int kinWord) {
   const int n = e->n, nc = e->mdNCons;
   double *x = e->x.as<double>(), *y = e->y.as<double>(), *z = e->z.as<double>();
   double *vx = e->mdV.as<double>(), *vy = vx + n, *vz = vy + n;
-  const double *fx = e->mdF.as<double>(), *fy = fx + n, *fz = fy + n;
   double *ddx = e->mdDd.as<double>(), *ddy = ddx + nc, *ddz = ddy + nc;
   long long *word = e->mdWord.as<long long>();
+  const double *rm = e->mdRmass.as<double>();
   const int g = grid_for(n, 256);
+  ForceSum fs;
+  MDB_TRY(md_force_parts(e, fs, s));
+  MdKin kin{};
+  if (kinWord >= 0)
+    kin = {e->mdMass.as<double>(), 4611686018427387904.0 / (double)(n > 0 ? n : 1),
+           word + kinWord, word};
+  if (!e->mdTri || e->mdNTri < n)
+    MDB_LAUNCH(k_vv_stage2, g, 256, 0, s, n, e->mdDt, fs, rm, vx, vy, vz,
+               e->mdTri ? e->mdNAt.as<int>() : nullptr);
   if (e->mdTri) {
-    if (e->mdNTri < n)
-      MDB_LAUNCH(k_vv_kick, g, 256, 0, s, n, e->mdDt, fx, fy, fz, e->mdRmass.as<double>(), vx,
-                 vy, vz, e->mdNAt.as<int>());
     MDB_LAUNCH(k_tri_stage2, grid_for(e->mdNMol, 128), 128, 0, s, e->mdNMol, BOXES(e), e->mdDt,
-               e->mdTol / e->mdDt, e->mdMaxCycle, e->mdTriAtoms.as<int4>(), fx, fy, fz,
-               e->mdRmass.as<double>(), x, y, z, vx, vy, vz,
-               reinterpret_cast<int *>(word + W_SHAKE));
-  } else {
-    MDB_LAUNCH(k_vv_kick, g, 256, 0, s, n, e->mdDt, fx, fy, fz, e->mdRmass.as<double>(), vx, vy,
-               vz, nullptr);
-  }
-  if (nc > 0 && !e->mdTri) {
+               e->mdTol / e->mdDt, e->mdMaxCycle, e->mdTriAtoms.as<int4>(), fs, rm, x, y, z, vx,
+               vy, vz, reinterpret_cast<int *>(word + W_SHAKE));
+  } else if (nc > 0) {
     // stage 2 takes the constraint vectors at the new positions
     MDB_LAUNCH(k_cons_vectors, grid_for(nc, 256), 256, 0, s, nc, BOXES(e), e->mdCa.as<int>(),
                e->mdCb.as<int>(), x, y, z, ddx, ddy, ddz);
@@ -1047,20 +1224,24 @@ int md_stage2(mdbas_nb_engine *e, cudaStream_t s, bool kin, double tauT, double 
                                        : k_shake_velocities<kMolMaxAtoms, kMolMaxCons>;
     MDB_LAUNCH(rattle, grid_for(e->mdNMol, 128), 128, 0, s, e->mdNMol, e->mdDt,
                e->mdTol / e->mdDt, e->mdMaxCycle, e->mdMol.as<int>(), e->mdCa.as<int>(),
-               e->mdCb.as<int>(), ddx, ddy, ddz, e->mdRmass.as<double>(), e->mdNAt.as<int>(), vx,
-               vy, vz, reinterpret_cast<int *>(word + W_SHAKE));
+               e->mdCb.as<int>(), ddx, ddy, ddz, rm, e->mdNAt.as<int>(), vx, vy, vz,
+               reinterpret_cast<int *>(word + W_SHAKE));
   }
-  const bool thermo = tauT > 0.;
-  if (kin || thermo) {
-    MDB_CUDA(cudaMemsetAsync(word + W_KIN, 0, sizeof(long long), s));
-    MDB_LAUNCH(k_kinetic, g, 256, 0, s, n, e->mdMass.as<double>(), vx, vy, vz,
-               4611686018427387904.0 / (double)(n > 0 ? n : 1), word + W_KIN, word + W_FLAGS);
-  }
-  if (thermo)
-    MDB_LAUNCH(k_berendsen, g, 256, 0, s, n, e->mdDt / tauT, kinTemp0, word + W_KIN, vx, vy,
-               vz);
-  // positions back into the box (image_update, src/integrate.c:1626)
-  MDB_LAUNCH(k_wrap, g, 256, 0, s, n, BOXES(e), x, y, z);
+  MDB_LAUNCH(k_kin_wrap, g, 256, 0, s, n, BOXES(e), x, y, z, vx, vy, vz, kin);
+  return MDBAS_NB_OK;
+}
+
+// The bath of a step; kin null without one.
+MdScale md_scale(const mdbas_nb_engine *e, double tauT, double kinTemp0, int kinWord) {
+  if (!(tauT > 0.)) return MdScale{};
+  return MdScale{e->mdWord.as<long long>() + kinWord, e->mdDt / tauT, kinTemp0};
+}
+
+int md_scale_velocities(mdbas_nb_engine *e, cudaStream_t s, const MdScale &sc) {
+  const int n = e->n;
+  double *vx = e->mdV.as<double>();
+  if (sc.kin)
+    MDB_LAUNCH(k_berendsen, grid_for(n, 256), 256, 0, s, n, sc, vx, vx + n, vx + 2 * (size_t)n);
   return MDBAS_NB_OK;
 }
 
@@ -1170,27 +1351,36 @@ int md_capture_steps(mdbas_nb_engine *e, int K, double tauT, double kinTemp0,
   const bool prune = md_prune_on(e);
   for (int k = 0; k < K; ++k) {
     g_launch_counter = &cc.main;
-    MDB_TRY(md_stage1(e, cs));
-    MDB_TRY(md_fork_terms(e, cs));
-    // the rebuild and prune decisions, on the device
     cudaStreamCaptureStatus cst;
     cudaGraph_t capG = nullptr;
     MDB_CUDA(cudaStreamGetCaptureInfo(cs, &cst, nullptr, &capG, nullptr, nullptr));
     // (a handle that no conditional node uses makes the graph invalid: the
-    // prune handle exists only with pruning on, else k_decide leaves it alone)
-    cudaGraphConditionalHandle hB, hP;
-    MDB_CUDA(cudaGraphConditionalHandleCreate(&hB, capG, 0, cudaGraphCondAssignDefault));
-    hP = hB;
+    // prune handle exists only with pruning on, else decide() leaves it alone)
+    MdDecide d{};
+    MDB_CUDA(cudaGraphConditionalHandleCreate(&d.hB, capG, 0, cudaGraphCondAssignDefault));
+    d.hP = d.hB;
     if (prune)
-      MDB_CUDA(cudaGraphConditionalHandleCreate(&hP, capG, 0, cudaGraphCondAssignDefault));
-    if (e->mdListUpdate == 0 || prune) MDB_TRY(md_max_disp(e, cs));
-    MDB_LAUNCH(k_decide, 1, 32, 0, cs, hB, hP,
-               reinterpret_cast<const unsigned long long *>(word + W_DISP),
-               reinterpret_cast<const unsigned long long *>(word + W_DISP2), half2, halfIn2,
-               e->mdListUpdate, prune ? 1 : 0, word + W_STEP);
+      MDB_CUDA(cudaGraphConditionalHandleCreate(&d.hP, capG, 0, cudaGraphCondAssignDefault));
+    d.half2 = half2;
+    d.halfIn2 = halfIn2;
+    d.update = e->mdListUpdate;
+    d.prune = prune ? 1 : 0;
+    // the kinetic-energy words take turns: this step's is cleared while the
+    // step before, which leaves the scaling of its velocities to this one's
+    // stage 1, is still recorded
+    d.kin = k & 1 ? W_KIN2 : W_KIN;
+    const int before = k & 1 ? W_KIN : W_KIN2;
+    // stage 1 with the rebuild and prune decisions, on the device
+    MdDisp disp = md_disp(e);
+    disp.active = 1;
+    disp.d = d;
+    MDB_TRY(md_stage1(e, cs, k > 0 ? md_scale(e, tauT, kinTemp0, before) : MdScale{}, disp));
+    if (!disp.xb) MDB_LAUNCH(k_decide, 1, 32, 0, cs, d, word);
+    if (k > 0) MDB_TRY(md_join(e, BR_SIDE, cs));
+    MDB_TRY(md_fork_terms(e, cs));
     cudaGraph_t body;
     cudaGraphNode_t node;
-    MDB_TRY(md_add_if(cs, hB, &body, &node));
+    MDB_TRY(md_add_if(cs, d.hB, &body, &node));
     long long bodyCount = 0;
     MDB_TRY(md_capture_rebuild_body(e, body, &bodyCount));
     cc.body = bodyCount;
@@ -1199,7 +1389,7 @@ int md_capture_steps(mdbas_nb_engine *e, int K, double tauT, double kinTemp0,
     g_launch_counter = &cc.main;
     MDB_TRY(md_refresh_cluster(e, cs));
     if (prune) {
-      MDB_TRY(md_add_if(cs, hP, &body, &node));
+      MDB_TRY(md_add_if(cs, d.hP, &body, &node));
       long long pruneCount = 0;
       MDB_TRY(md_capture_prune_body(e, body, &pruneCount));
       cc.prune = pruneCount;
@@ -1208,12 +1398,14 @@ int md_capture_steps(mdbas_nb_engine *e, int K, double tauT, double kinTemp0,
       g_launch_counter = &cc.main;
     }
     MDB_TRY(md_forces_cluster(e, cs));
-    MDB_TRY(md_stage2(e, cs, true, tauT, kinTemp0));
-    MDB_LAUNCH(k_md_row, 1, 32, 0, cs, e->mdRows.as<long long>() + kRowWords * (size_t)k,
-               e->cl.acc.as<long long>(), word + W_KIN, md_bonded_fix(e), md_kspace_fix(e),
-               word + W_FLAGS);
+    MDB_TRY(md_stage2(e, cs, d.kin));
+    if (k == K - 1) MDB_TRY(md_scale_velocities(e, cs, md_scale(e, tauT, kinTemp0, d.kin)));
+    MDB_TRY(md_fork(e, BR_SIDE, cs));
+    MDB_LAUNCH(k_md_row, 1, 32, 0, e->mdBranch[BR_SIDE],
+               e->mdRows.as<long long>() + kRowWords * (size_t)k, e->cl.acc.as<long long>(),
+               word + d.kin, md_bonded_fix(e), md_kspace_fix(e), word);
   }
-  return MDBAS_NB_OK;
+  return md_join(e, BR_SIDE, cs);
 }
 
 int md_capture(mdbas_nb_engine *e, int K, double targetTemp, double tauT, double kinTemp0) {
@@ -1256,7 +1448,7 @@ int md_capture(mdbas_nb_engine *e, int K, double targetTemp, double tauT, double
   e->mdGraphTau = tauT;
   e->mdGraphTemp = targetTemp;
   e->mdGraphStale = false;
-  e->mdGraphMainK = cc.main / K;
+  e->mdGraphMainK = cc.main;
   e->mdGraphBodyK = cc.body;
   e->mdGraphPruneK = cc.prune;
   return MDBAS_NB_OK;
@@ -1304,8 +1496,8 @@ int md_run_graph(mdbas_nb_engine *e, int chunks, int energyEvery, double targetT
     const long long step0 = e->mdSteps;
     MDB_CUDA(cudaMemcpyAsync(word + W_STEP, &step0, sizeof(long long), cudaMemcpyHostToDevice,
                              s));
-    MDB_CUDA(cudaMemsetAsync(word + W_BUILDS, 0, sizeof(long long), s));
-    MDB_CUDA(cudaMemsetAsync(word + W_PRUNES, 0, sizeof(long long), s));
+    for (const int k : {W_BUILDS, W_PRUNES, W_DISP, W_DISP2, W_DONE})
+      MDB_CUDA(cudaMemsetAsync(word + k, 0, sizeof(long long), s));
     MDB_CUDA(cudaMemsetAsync(e->cl.sticky.p, 0, sizeof(long long), s));
     MD_TRY(md_snapshot(e, false));
     MDB_CUDA(cudaGraphLaunch(e->mdExec, s));
@@ -1315,7 +1507,7 @@ int md_run_graph(mdbas_nb_engine *e, int chunks, int energyEvery, double targetT
     MDB_CUDA(cudaMemcpyAsync(rows.data(), e->mdRows.p, sizeof(long long) * rows.size(),
                              cudaMemcpyDeviceToHost, s));
     MDB_CUDA(cudaStreamSynchronize(s));
-    e->launches += e->mdGraphMainK * K + e->mdGraphBodyK * w[W_BUILDS] +
+    e->launches += e->mdGraphMainK + e->mdGraphBodyK * w[W_BUILDS] +
                    e->mdGraphPruneK * w[W_PRUNES];
     if (sticky & CL_NONFINITE) {
       set_last_status(MDBAS_NB_ERR_NONFINITE, "non-finite positions during dynamics");
@@ -1619,13 +1811,16 @@ int mdbas_nb_engine_md_run(mdbas_nb_engine *e, int nSteps, int energyEvery, doub
   }
   for (int step = done; step < nSteps; ++step) {
     const long long gstep = e->mdSteps + 1;
-    MD_TRY(md_stage1(e, s));
+    const MdDisp disp = md_disp(e);
+    if (disp.xb)
+      for (const int k : {W_DISP, W_DISP2})
+        MDB_CUDA(cudaMemsetAsync(word + k, 0, sizeof(long long), s));
+    MD_TRY(md_stage1(e, s, MdScale{}, disp));
     // list: fixed cadence or half-skin displacement; inner list: a rebuild
-    // or half the prune buffer since the last prune (k_decide's rules)
+    // or half the prune buffer since the last prune (decide()'s rules)
     const bool prune = md_prune_on(e);
     double d2 = 0., p2 = 0.;
     if (e->mdListUpdate == 0 || prune) {
-      MD_TRY(md_max_disp(e, s));
       unsigned long long bits[2] = {0, 0};
       MDB_CUDA(cudaMemcpyAsync(&bits[0], word + W_DISP, sizeof(bits[0]), cudaMemcpyDeviceToHost,
                                s));
@@ -1640,9 +1835,14 @@ int mdbas_nb_engine_md_run(mdbas_nb_engine *e, int nSteps, int energyEvery, doub
     if (e->cfg.precision == 1) MD_TRY(mdbas_nb_engine_refresh(e));
     if (prune && (rebuild || p2 > halfIn2)) MD_TRY(md_prune_sync(e));
     MD_TRY(mdbas_nb_engine_compute(e));
-    MD_TRY(md_forces(e, s));
+    MD_TRY(md_kspace_terms(e, s));
+    MD_TRY(md_bonded_terms(e, s));
     const bool wantE = energies && energyEvery > 0 && (gstep % energyEvery) == 0;
-    MD_TRY(md_stage2(e, s, wantE, tauT, kinTemp0));
+    const MdScale sc = md_scale(e, tauT, kinTemp0, W_KIN);
+    const bool wantKin = wantE || sc.kin;
+    if (wantKin) MDB_CUDA(cudaMemsetAsync(word + W_KIN, 0, sizeof(long long), s));
+    MD_TRY(md_stage2(e, s, wantKin ? W_KIN : -1));
+    MD_TRY(md_scale_velocities(e, s, sc));
     if (wantE) {
       long long kfix = 0;
       MDB_CUDA(cudaMemcpyAsync(&kfix, word + W_KIN, sizeof(kfix), cudaMemcpyDeviceToHost, s));
