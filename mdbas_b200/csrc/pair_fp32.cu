@@ -727,9 +727,13 @@ constexpr int kHIt = 8;  // steps per staged chunk
 // Two copies of each step's data: in order (half A in .x, B in .y) for lanes
 // with i atom 0-3, swapped for lanes with i atom 4-7, so that in the first
 // round of the j-force reduce-scatter every lane keeps .x and passes .y.
+// The copies are padded apart so that the four atoms of a step in one order and
+// the four in the other, which a warp reads at once, fall into the eight
+// 16-byte bank groups (10^6 atoms, full list: 2.82 ms without, 2.76 with).
 struct HalfStage {
-  float4 jd[2][kHIt * 4 * 3];  // [order][step][half atom]: (x,x,y,y), (z,z,q,q), (eps,eps,sig,sig)
-  int4 mj[2][kHIt];            // [order][step]: masks of the two halves, their first slots
+  // [order][step][half atom]: (x,x,y,y), (z,z,q,q), (eps,eps,sig,sig)
+  float4 jd[2][kHIt * 4 * 3 + 4];
+  int4 mj[2][kHIt + 1];        // [order][step]: masks of the two halves, their first slots
   float sh[kHIt][8];           // per step: sxA, sxB, syA, syB, szA, szB
   int2 js[kHIt];               // per step: first slot of half A, of half B
   uint2 mk[kHIt];              // per step: masks of half A, of half B
