@@ -104,9 +104,9 @@ struct mdbas_nb_engine {
   cudaGraph_t mdGraph = nullptr;
   cudaGraphExec_t mdExec = nullptr;
   cudaStream_t mdCapStream = nullptr, mdSideStream = nullptr;
-  // branches of the captured step (md.cu: MdBranch) and their fork/join events
-  cudaStream_t mdBranch[4] = {};
-  cudaEvent_t mdForkEv = nullptr, mdJoinEv[4] = {};
+  // branches of the captured step (md.cu: MdBranch) and their fork and join events
+  cudaStream_t mdBranch[2] = {};
+  cudaEvent_t mdForkEv = nullptr, mdClearEv = nullptr, mdJoinEv[2] = {};
   mdbas::DBuf mdRows, mdSnap;
 };
 

@@ -1138,10 +1138,13 @@ int md_prune_sync(mdbas_nb_engine *e) {
 // pair kernel of 10,000 atoms leaves most of the chip idle for its 52 us, and
 // the 16 kernels of its SPME take 105: a step of flexible chains with SPME
 // 196 -> 160 us; of 96,000 atoms of water (the exclusions' 11 us) 441 -> 434.
-// With the small kernels folded into the half kicks besides, 149 and 399.
-// BR_SIDE takes what leaves the step's own path free: the record of a step
-// (during the next one's stage 1) and the clearing of the force words.
-enum MdBranch { BR_KSPACE = 0, BR_BONDED = 1, BR_EXCL = 2, BR_SIDE = 3 };
+// With the small kernels folded into the half kicks besides, 149 and 415.
+// BR_SIDE takes, one after the other, what leaves the step's own path free: the
+// record of a step (during the next one's stage 1), the clearing of the force
+// words, the bonded terms and the exclusions.  (A branch each: no faster, and
+// the graph of 20 steps took 6.6 ms to instantiate with SPME
+// and bonded terms, 3.7 without, against 5.2 and 2.6.)
+enum MdBranch { BR_KSPACE = 0, BR_SIDE = 1 };
 
 int md_fork(mdbas_nb_engine *e, MdBranch b, cudaStream_t s) {
   MDB_CUDA(cudaEventRecord(e->mdForkEv, s));
@@ -1155,18 +1158,17 @@ int md_join(mdbas_nb_engine *e, MdBranch b, cudaStream_t s) {
   return MDBAS_NB_OK;
 }
 
-// The captured step's branches that start at the new positions.
+// What of a captured step starts at the new positions; mdClearEv: facc and
+// acc are clear.
 int md_fork_terms(mdbas_nb_engine *e, cudaStream_t s) {
   if (e->kspaceKind != 0) {
     MDB_TRY(md_fork(e, BR_KSPACE, s));
     MDB_TRY(md_kspace_terms(e, e->mdBranch[BR_KSPACE]));
   }
-  if (e->bonded.nTerms() > 0) {
-    MDB_TRY(md_fork(e, BR_BONDED, s));
-    MDB_TRY(md_bonded_terms(e, e->mdBranch[BR_BONDED]));
-  }
   MDB_TRY(md_fork(e, BR_SIDE, s));
-  return cluster_clear(e->cl, e->mdBranch[BR_SIDE]);
+  MDB_TRY(cluster_clear(e->cl, e->mdBranch[BR_SIDE]));
+  MDB_CUDA(cudaEventRecord(e->mdClearEv, e->mdBranch[BR_SIDE]));
+  return md_bonded_terms(e, e->mdBranch[BR_SIDE]);
 }
 
 // Forces of a captured step on the current layout (refreshed by the caller):
@@ -1174,15 +1176,14 @@ int md_fork_terms(mdbas_nb_engine *e, cudaStream_t s) {
 int md_forces_cluster(mdbas_nb_engine *e, cudaStream_t s) {
   ClusterWork &w = e->cl;
   const int n = e->n;
-  MDB_TRY(md_join(e, BR_SIDE, s));  // facc and acc are clear
-  MDB_TRY(md_fork(e, BR_EXCL, s));
+  MDB_CUDA(cudaStreamWaitEvent(s, e->mdClearEv, 0));
+  MDB_TRY(md_fork(e, BR_SIDE, s));
   MDB_TRY(excl_fix_launch(w, n, e->pp, e->exclStartSym.as<int>(), e->exclFlatSym.as<int>(),
                           e->x.as<double>(), e->y.as<double>(), e->z.as<double>(),
-                          e->q.as<double>(), e->mdBranch[BR_EXCL]));
+                          e->q.as<double>(), e->mdBranch[BR_SIDE]));
   MDB_TRY(pair_fp32_launch(w, e->pp, e->grid, e->block, s, e->variant));
-  MDB_TRY(md_join(e, BR_EXCL, s));
+  MDB_TRY(md_join(e, BR_SIDE, s));
   if (e->kspaceKind != 0) MDB_TRY(md_join(e, BR_KSPACE, s));
-  if (e->bonded.nTerms() > 0) MDB_TRY(md_join(e, BR_BONDED, s));
   return MDBAS_NB_OK;
 }
 
@@ -1416,9 +1417,8 @@ int md_capture(mdbas_nb_engine *e, int K, double targetTemp, double tauT, double
     MDB_CUDA(cudaStreamCreateWithFlags(&e->mdSideStream, cudaStreamNonBlocking));
   for (cudaStream_t &b : e->mdBranch)
     if (!b) MDB_CUDA(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
-  if (!e->mdForkEv) MDB_CUDA(cudaEventCreateWithFlags(&e->mdForkEv, cudaEventDisableTiming));
-  for (cudaEvent_t &ev : e->mdJoinEv)
-    if (!ev) MDB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  for (cudaEvent_t *ev : {&e->mdForkEv, &e->mdClearEv, &e->mdJoinEv[0], &e->mdJoinEv[1]})
+    if (!*ev) MDB_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
   MDB_TRY(e->mdRows.ensure(sizeof(long long) * kRowWords * (size_t)K));
   // everything the capture reads from the host must be final: finish the
   // engine stream's work first
@@ -1566,12 +1566,10 @@ void mdbas::md_release(mdbas_nb_engine *e) {
     if (b) cudaStreamDestroy(b);
     b = nullptr;
   }
-  for (cudaEvent_t &ev : e->mdJoinEv) {
-    if (ev) cudaEventDestroy(ev);
-    ev = nullptr;
+  for (cudaEvent_t *ev : {&e->mdForkEv, &e->mdClearEv, &e->mdJoinEv[0], &e->mdJoinEv[1]}) {
+    if (*ev) cudaEventDestroy(*ev);
+    *ev = nullptr;
   }
-  if (e->mdForkEv) cudaEventDestroy(e->mdForkEv);
-  e->mdForkEv = nullptr;
 }
 
 extern "C" {
