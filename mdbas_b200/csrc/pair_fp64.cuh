@@ -1,4 +1,4 @@
-// pair_fp64.cuh -- plain FP64 pair kernels (MDBas's loops, one thread per i).
+// pair_fp64.cuh -- plain FP64 pair kernels over MDBas's list.
 #pragma once
 
 #include "common.cuh"
