@@ -1417,8 +1417,21 @@ int cluster_build(ClusterWork &w, int n, int nRep, const DevBox *boxes, const in
   bool sameGrid = nRep == w.nRep && w.atomOffH.size() == (size_t)nRep + 1;
   for (int r = 0; sameGrid && r < nRep; ++r)
     sameGrid = same_geom(geoms[r], w.geomH[r]) && atomOff[r + 1] == w.atomOffH[r + 1];
-  // The captured form cannot upload tables or grow buffers.
-  if (!sync && (!sameGrid || slotCap > w.slotCap || w.entryCap == 0)) return MDBAS_NB_ERR_STATE;
+  // The form that does not wait cannot upload tables or grow buffers: they
+  // have to hold the capacities already (the dynamics raise those of a list
+  // that was outgrown; an allocation may have failed in between).
+  const auto holds = [](const DBuf &b, size_t item, long long count) {
+    return b.bytes >= item * (size_t)count;
+  };
+  if (!sync &&
+      (!sameGrid || slotCap > w.slotCap || w.entryCap == 0 ||
+       !holds(w.facc, 3 * sizeof(long long), w.slotCap) ||
+       !holds(w.entries, sizeof(CPairEntry), w.entryCap) ||
+       !holds(w.masks, sizeof(uint2), w.entryCap) || !holds(w.items, sizeof(int4), w.itemCap) ||
+       !holds(w.entriesIn, sizeof(HalfEntry), 2 * w.entryCap) ||
+       !holds(w.masksIn, sizeof(unsigned), 2 * w.entryCap) ||
+       !holds(w.itemsIn, sizeof(int4), w.itemCap)))
+    return MDBAS_NB_ERR_STATE;
 
   // Per-replica tables, rebuilt when any grid changes: Morton rank of each
   // (cx, cy) cell as a global column, and each column's (cx, cy).
