@@ -1494,10 +1494,12 @@ int md_run_graph(mdbas_nb_engine *e, int chunks, int energyEvery, double targetT
   int growths = 0;
   for (int c = 0; c < chunks;) {
     const long long step0 = e->mdSteps;
+    // every word starts over, the error bits too: a chunk is checked before
+    // the next one is launched, and what a chunk that is taken back raised
+    // does not count
+    MDB_CUDA(cudaMemsetAsync(word, 0, sizeof(long long) * W_COUNT, s));
     MDB_CUDA(cudaMemcpyAsync(word + W_STEP, &step0, sizeof(long long), cudaMemcpyHostToDevice,
                              s));
-    for (const int k : {W_BUILDS, W_PRUNES, W_DISP, W_DISP2, W_DONE})
-      MDB_CUDA(cudaMemsetAsync(word + k, 0, sizeof(long long), s));
     MDB_CUDA(cudaMemsetAsync(e->cl.sticky.p, 0, sizeof(long long), s));
     MD_TRY(md_snapshot(e, false));
     MDB_CUDA(cudaGraphLaunch(e->mdExec, s));
@@ -1509,14 +1511,17 @@ int md_run_graph(mdbas_nb_engine *e, int chunks, int energyEvery, double targetT
     MDB_CUDA(cudaStreamSynchronize(s));
     e->launches += e->mdGraphMainK + e->mdGraphBodyK * w[W_BUILDS] +
                    e->mdGraphPruneK * w[W_PRUNES];
-    if (sticky & CL_NONFINITE) {
+    const bool grow = (sticky & CL_OVERFLOW) && growths < 3;
+    if ((sticky & CL_NONFINITE) && !grow) {
       set_last_status(MDBAS_NB_ERR_NONFINITE, "non-finite positions during dynamics");
       return MDBAS_NB_ERR_NONFINITE;
     }
     if (sticky & CL_OVERFLOW) {
       // a rebuild inside the chunk outgrew the pair list: go back to the
-      // chunk's start, enlarge the list and capture again
-      if (++growths > 3) return MDBAS_NB_ERR_CAPACITY;
+      // chunk's start, enlarge the list and capture again.  This comes before
+      // every other error: the steps after that rebuild had an empty list
+      if (!grow) return MDBAS_NB_ERR_CAPACITY;
+      ++growths;
       MD_TRY(md_snapshot(e, true));
       e->cl.entryCap = (long long)(e->cl.entryCap * 1.5) + 4096;
       e->cl.itemCap = (long long)(e->cl.itemCap * 1.5) + 1024;
