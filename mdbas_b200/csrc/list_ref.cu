@@ -174,20 +174,29 @@ __device__ __forceinline__ int stencil_cell(int l, int ix, int iy, int iz, int n
   return jx + nx * (jy + ny * jz);
 }
 
-// Candidate chunks of every cell, one warp per cell: chunkOff[l], the first
-// chunk of stencil cell l (its atoms in runs of 32), chunkOff[cellCheck] the
-// total, and chunkBase[c], the first position of chunk c.  A total beyond
+// A cell's row in the candidate tables: its number, or, where there are more
+// cells than atoms (byStart), the position of its first atom, which no other
+// occupied cell has.  So the tables have min(cells, atoms) rows: a droplet of
+// 3,000 atoms in a 2,000 A box has 2.9 million cells.
+__device__ __forceinline__ size_t table_row(int byStart, int cell, const int *cellStart) {
+  return byStart ? cellStart[cell] : cell;
+}
+
+// Candidate chunks of every occupied cell, one warp per cell: chunkOff[l], the
+// first chunk of stencil cell l (its atoms in runs of 32), chunkOff[cellCheck]
+// the total, and chunkBase[c], the first position of chunk c.  A total beyond
 // stride raises FLAG_CELL and goes to *need.
 __global__ void __launch_bounds__(32 * kListWarps)
-k_lc_chunks(int ncell, int nx, int ny, int nz, int cellCheck, int stride,
+k_lc_chunks(int ncell, int nx, int ny, int nz, int cellCheck, int stride, int byStart,
             const int *__restrict__ cellStart, int *__restrict__ chunkOff,
             int *__restrict__ chunkBase, int *__restrict__ flags, int *__restrict__ need) {
   const int lane = threadIdx.x & 31;
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (k >= ncell) return;
+  if (k >= ncell || cellStart[k] == cellStart[k + 1]) return;
   const int ix = k % nx, iy = (k / nx) % ny, iz = k / (nx * ny);
-  int *off = chunkOff + (size_t)k * (cellCheck + 1);
-  int *base = chunkBase + (size_t)k * stride;
+  const size_t row = table_row(byStart, k, cellStart);
+  int *off = chunkOff + row * (cellCheck + 1);
+  int *base = chunkBase + row * stride;
   int run = 0;
   for (int l0 = 0; l0 < cellCheck; l0 += 32) {
     const int l = l0 + lane;
@@ -225,17 +234,20 @@ k_lc_chunks(int ncell, int nx, int ny, int nz, int cellCheck, int stride,
 // consecutive positions that lies in one cell; chunks of the own cell before
 // the run hold no candidate.  All pairs: chunk c is atoms 32c .. 32c + 31.
 struct ChunkMap {
-  int linkCells, n, stride, cellCheck, ncell, nlc[3];
+  int linkCells, n, stride, cellCheck, ncell, byStart, nlc[3];
   const int *cellStart, *cellOf, *order, *posOf, *chunkOff, *chunkBase;
 
   __device__ __forceinline__ int atoms() const { return linkCells ? cellStart[ncell] : n; }
   __device__ __forceinline__ int atom(int p) const { return linkCells ? order[p] : p; }
+  __device__ __forceinline__ const int *offsets(int cell) const {
+    return chunkOff + table_row(byStart, cell, cellStart) * (cellCheck + 1);
+  }
   __device__ __forceinline__ void range(int p, int cell, int &first, int &last) const {
     const int g0 = p & ~(kGroup - 1);
     if (linkCells) {
       const int s = cellStart[cell];
       first = (max(g0, s) + 1 - s) >> 5;
-      last = chunkOff[(size_t)cell * (cellCheck + 1) + cellCheck];
+      last = offsets(cell)[cellCheck];
     } else {
       first = (g0 + 1) >> 5;
       last = (n + 31) >> 5;
@@ -313,7 +325,7 @@ k_lc_masks(int p0, int p1, DevBox b, ChunkMap map, double cutnb2, float rl2, flo
     unsigned *rows = masks + (size_t)(p - p0) * map.stride;
     // this warp's piece of the chunks, from the first that holds a position
     // after p
-    const int *off = map.chunkOff + (size_t)k * (map.cellCheck + 1);
+    const int *off = map.offsets(k);
     const int cFirst = max((p + 1 - map.cellStart[k]) >> 5, (int)blockIdx.y * kPiece);
     const int cLast = min(off[map.cellCheck], (int)(blockIdx.y + 1) * kPiece);
     if (cFirst >= cLast) {
@@ -537,8 +549,7 @@ k_list_count(int p0, int p1, ChunkMap map, const int *__restrict__ exclStart,
                               kMaxRatio];
     if (l < 0 || l >= map.cellCheck) continue;
     const int o = map.posOf[j] - map.cellStart[kj];
-    atomicAnd(row + map.chunkOff[(size_t)cell * (map.cellCheck + 1) + l] + (o >> 5),
-              ~(1u << (o & 31)));
+    atomicAnd(row + map.offsets(cell)[l] + (o >> 5), ~(1u << (o & 31)));
   }
   __syncwarp();
   int first, last, total = 0;
@@ -564,7 +575,9 @@ k_list_fill(int p0, int p1, ChunkMap map, const unsigned *__restrict__ masks,
   int *const b = buf[threadIdx.x >> 5];
   const unsigned *row = masks + (size_t)(p - p0) * map.stride;
   const int cell = map.linkCells ? map.cellOf[map.order[p]] : 0;
-  const int *bases = map.chunkBase + (size_t)cell * map.stride;
+  const int *bases =
+      map.linkCells ? map.chunkBase + table_row(map.byStart, cell, map.cellStart) * map.stride
+                    : nullptr;
   int first, last;
   map.range(p, cell, first, last);
   int *out = list + off[p];
@@ -692,6 +705,7 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
     map.ncell = w.ncell;
     for (int d = 0; d < 3; ++d) map.nlc[d] = w.nlc[d];
     map.cellCheck = LINK_STENCIL_COUNT[ratio - 1];
+    map.byStart = w.ncell > n;
     // chunks per cell of evenly spread atoms with room for fluctuations; a
     // denser cell reports what it needs and the build is made again
     const double per = (double)n / w.ncell;
@@ -703,6 +717,7 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
   }
   MDB_TRY(w.scanTmp.ensure(std::max(scan_tmp_bytes(w.ncell + 1), scan_tmp_bytes(n + 1))));
   const int ncell = w.ncell;
+  const size_t tableRows = std::min(ncell, n);
   if (linkCells) {
     MDB_TRY(w.xu.ensure(sizeof(double) * n));
     MDB_TRY(w.yu.ensure(sizeof(double) * n));
@@ -716,7 +731,7 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
     // counts and fill marks side by side: cleared together
     MDB_TRY(w.cellCount.ensure(sizeof(int) * 2 * (size_t)(ncell + 1)));
     MDB_TRY(w.cellStart.ensure(sizeof(int) * (ncell + 2)));
-    MDB_TRY(w.chunkOff.ensure(sizeof(int) * (size_t)ncell * (map.cellCheck + 1)));
+    MDB_TRY(w.chunkOff.ensure(sizeof(int) * tableRows * (map.cellCheck + 1)));
   }
 
   for (int attempt = 0;; ++attempt) {
@@ -725,7 +740,7 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
     int exactOnly = 0;
     if (linkCells) {
       int *count = w.cellCount.as<int>(), *fill = count + ncell + 1;
-      MDB_TRY(w.chunkBase.ensure(sizeof(int) * (size_t)ncell * map.stride));
+      MDB_TRY(w.chunkBase.ensure(sizeof(int) * tableRows * map.stride));
       map.cellStart = w.cellStart.as<int>();
       map.cellOf = w.cellOf.as<int>();
       map.order = w.order.as<int>();
@@ -752,8 +767,9 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
                  frozen, w.xs.as<double>(), w.ys.as<double>(), w.zs.as<double>(),
                  w.cs.as<float4>(), w.posOf.as<int>());
       MDB_LAUNCH(k_lc_chunks, grid_for(ncell, kListWarps), 32 * kListWarps, 0, s, ncell, w.nlc[0],
-                 w.nlc[1], w.nlc[2], map.cellCheck, map.stride, w.cellStart.as<int>(),
-                 w.chunkOff.as<int>(), w.chunkBase.as<int>(), flags, flags + 1);
+                 w.nlc[1], w.nlc[2], map.cellCheck, map.stride, map.byStart,
+                 w.cellStart.as<int>(), w.chunkOff.as<int>(), w.chunkBase.as<int>(), flags,
+                 flags + 1);
     } else {
       const double bx = b.a1, by = b.type == CUBIC ? b.a1 : b.b2,
                    bz = b.type == CUBIC ? b.a1 : b.c3;
