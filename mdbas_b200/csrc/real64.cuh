@@ -53,7 +53,8 @@ __constant__ static const double kExpC[12] = {  // 1 / k!, k = 2..13
 
 // erfc(x) exp(x^2) on [0, 6]: (x + 3) erfcx(x) is a polynomial of degree 18 in
 // (x - 3) / (x + 3) to a relative 1.9e-17 (fit_erfc.py: Chebyshev
-// interpolation in 70-digit arithmetic).
+// interpolation in 70-digit arithmetic).  The map is that of M. M. Shepherd and
+// J. G. Laframboise, Math. Comp. 36 (1981) 249, who take it over [0, inf).
 constexpr double kErfcxMax = 6.0;
 __device__ __forceinline__ double erfcx64(double x) {
   const double inv = rcp64(x + 3.0);
@@ -82,10 +83,12 @@ __device__ __forceinline__ double expm64(double u) {
 
 // exp(-(a2 + a2lo) r2) from a product in two parts (a2 + a2lo is alpha^2 to
 // twice the precision): a rounded x^2 would put an error of x^2 ulps on it.
+// a2lo r2 is less than half an ulp of u: it is added to what u's rounding left
+// out, not to u.
 __device__ __forceinline__ double expm64_product(double a2, double a2lo, double r2) {
   const double u = a2 * r2;
   const double g = expm64(u);
-  return fma(-g, fma(a2, r2, fma(a2lo, r2, -u)), g);
+  return fma(-g, fma(a2lo, r2, fma(a2, r2, -u)), g);
 }
 
 // 2 alpha / sqrt(pi), alpha^2 in two parts, and the switch's factor and
