@@ -171,18 +171,21 @@ constexpr int kPairBlocks = 6;    // blocks per SM
 // The sum of every block's v into acc[c], without the rounding of one FP64
 // addition after the other (a thousand blocks' would show in differences of
 // energies): multiples of 2^-10 and what is left of v, in multiples of 2^-60,
-// are added as integers, and the last block puts them together.  A sum too
-// large for that is added as it is.
+// are added as integers, and the last block puts them together.  What v holds
+// below 2^-60 (nothing from 2^-7 on; all of a weak pair's energy of 1e-19) and
+// sums too large for the integers are added as they are.
 __device__ __forceinline__ void exact_add(double *acc, int c, double v) {
   if (!(fabs(v) < 1e12)) {
     atomicAdd(acc + c, v);
     return;
   }
   const long long h = __double2ll_rn(v * 1024.);
-  const double rest = v - (double)h * (1. / 1024.);
+  double rest = v - (double)h * (1. / 1024.);
+  const long long l = __double2ll_rn(rest * 1152921504606846976.);
+  rest -= (double)l * (1. / 1152921504606846976.);
   red_add(reinterpret_cast<long long *>(acc + 8 + 2 * c), h);
-  red_add(reinterpret_cast<long long *>(acc + 9 + 2 * c),
-          __double2ll_rn(rest * 1152921504606846976.));
+  red_add(reinterpret_cast<long long *>(acc + 9 + 2 * c), l);
+  if (rest != 0.) atomicAdd(acc + c, rest);
 }
 __device__ __forceinline__ void exact_finish(double *acc, int c) {
   const long long h = __ldcg(reinterpret_cast<long long *>(acc + 8 + 2 * c));

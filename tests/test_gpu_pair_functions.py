@@ -12,7 +12,8 @@ rounding is at most 1 u):
   exp(-x^2) from the two-part product 3.2;
   an energy C q q exp erfcx / r: 11 + 3.2 + 1.5 and three products, 19;
   r dE/dr: the energy or the second term (less), and the sum, 20;
-  a force: that, 1/r^2 within 1, two products, 23.
+  a force: that, 1/r^2 within 1, two products, 23;
+  a sum over blocks: three additions more, 22 and 23.
 """
 import decimal
 import math
@@ -110,3 +111,21 @@ def test_pair_adjoint(gpu, alpha, cut_off):
           np.sqrt((d * d).mean()))
     assert np.abs(d).max() <= 19
 
+
+@pytest.mark.parametrize("q", [1.0, 2.0 ** -20])
+def test_single_pair_energy(gpu, q):
+    """The sum over blocks keeps the digits of one weak pair."""
+    alpha = 0.5
+    dist = np.array([1.0, 4.0, 7.5, 9.0, 10.5, 11.25, 12.0])
+    want = [x * D(q) * D(q) for x in _exact(dist, alpha)[0]]
+    work = [-x * D(r) * D(q) * D(q) for x, r in zip(_exact(dist, alpha)[1], dist)]
+    for r, e, w in zip(dist, want, work):
+        eng = _engine(_pairs(np.array([r]), q, q), alpha, 12.0)
+        eng.build()
+        eng.compute()
+        got = eng.energies()
+        eng.close()
+        assert got["n_pairs"] == 1
+        print(q, r, _off([got["elec_direct"]], [e]), _off([got["vir_direct"]], [w]))
+        assert abs(_off([got["elec_direct"]], [e])[0]) <= 22
+        assert abs(_off([got["vir_direct"]], [w])[0]) <= 23
