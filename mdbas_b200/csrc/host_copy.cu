@@ -49,6 +49,7 @@ constexpr int kSlots = 32;    // 16 MB page-locked at most
 constexpr int kPlainFirst = 8;
 constexpr int kHelpers = 3;
 constexpr size_t kManyFrom = (size_t)8 << 20;     // smaller transfers: one helper
+constexpr int kMaxSpans = 16;
 constexpr size_t kLookFrom = (size_t)128 << 10;   // smaller arrays: staged even if page-locked
 
 // Helper threads that run one job at a time; a job is a function every
@@ -276,12 +277,24 @@ void run(void *arg) {
   }
 }
 
-cudaError_t plain(const CopySpan &sp, cudaStream_t s) {
-  if (!sp.add) return cudaMemcpyAsync(sp.host, sp.dev, sp.bytes, cudaMemcpyDeviceToHost, s);
-  std::vector<double> h(sp.bytes / sizeof(double));
-  cudaError_t e = cudaMemcpyAsync(h.data(), sp.dev, sp.bytes, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) add(static_cast<double *>(sp.host), h.data(), h.size());
+// The plain way; what is added is added once all of the spans are there.
+cudaError_t plain(const CopySpan *spans, int count, cudaStream_t s) {
+  std::vector<std::vector<double>> h(count);
+  bool adds = false;
+  for (int k = 0; k < count; ++k)
+    if (spans[k].add) {
+      h[k].resize(spans[k].bytes / sizeof(double));
+      adds = true;
+    }
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < count && e == cudaSuccess; ++k)
+    e = cudaMemcpyAsync(spans[k].add ? h[k].data() : spans[k].host, spans[k].dev, spans[k].bytes,
+                        cudaMemcpyDeviceToHost, s);
+  if (!adds) return e;
+  const cudaError_t w = cudaStreamSynchronize(s);  // before h goes, in any case
+  if (e == cudaSuccess) e = w;
+  for (int k = 0; k < count && e == cudaSuccess; ++k)
+    if (spans[k].add) add(static_cast<double *>(spans[k].host), h[k].data(), h[k].size());
   return e;
 }
 
@@ -297,27 +310,20 @@ int copy_in(const CopySpan *spans, int count, cudaStream_t s) {
 
 namespace {
 
-int unpack(const CopySpan *spans, int count, cudaStream_t s) {
-  CopySpan staged[16];
-  int ns = 0;
+// With the pool's slots, or without (p null).
+int unpack(const CopySpan *spans, int count, cudaStream_t s, Pool *p) {
+  CopySpan staged[kMaxSpans], direct[kMaxSpans];
+  int ns = 0, nd = 0;
   size_t bytes = 0;
   bool adds = false;
-  if (count > 16) return MDBAS_NB_ERR_ARG;
-  Pool &p = pool();
-  std::unique_lock<std::mutex> lk(p.busy, std::try_to_lock);
-  if (lk.owns_lock() && p.plain < kPlainFirst) {
-    ++p.plain;
-    lk.unlock();
-  }
   for (int k = 0; k < count; ++k) {
     if (spans[k].bytes == 0) continue;
-    if (lk.owns_lock() &&
-        (spans[k].add || spans[k].bytes < kLookFrom || pageable(spans[k].host))) {
+    if (p && (spans[k].add || spans[k].bytes < kLookFrom || pageable(spans[k].host))) {
       adds |= spans[k].add;
       bytes += spans[k].bytes;
       staged[ns++] = spans[k];
     } else {
-      MDB_CUDA(plain(spans[k], s));
+      direct[nd++] = spans[k];
     }
   }
   std::vector<Piece> pieces;
@@ -326,20 +332,21 @@ int unpack(const CopySpan *spans, int count, cudaStream_t s) {
   const int n = (int)chunks.size();
   int dev = 0;
   if (n > 0) MDB_CUDA(cudaGetDevice(&dev));
-  if (n > 0 && !p.ready(std::min(n, kSlots), dev)) {  // no page-locked memory left
-    for (int k = 0; k < ns; ++k) MDB_CUDA(plain(staged[k], s));
-  } else if (n > 0) {
+  if (n > 0 && !p->ready(std::min(n, kSlots), dev))  // no page-locked memory left
+    return unpack(spans, count, s, nullptr);
+  if (nd > 0) MDB_CUDA(plain(direct, nd, s));
+  if (n > 0) {
     Transfer t(n);
-    t.p = &p;
+    t.p = p;
     t.s = s;
     t.device = dev;
     t.pieces.swap(pieces);
     t.chunks.swap(chunks);
     for (int c = 0; c < std::min(n, kSlots); ++c) issue_marked(t, c);
     const int helpers = adds || n == 1 ? 0 : bytes < kManyFrom ? 1 : kHelpers;
-    if (helpers > 0) p.helpers.start(helpers, run, &t);
+    if (helpers > 0) p->helpers.start(helpers, run, &t);
     run(&t);
-    if (helpers > 0) p.helpers.finish();
+    if (helpers > 0) p->helpers.finish();
     if (const int e = t.err.load())
       return cuda_fail((cudaError_t)e, "copy_out", __FILE__, __LINE__);
   }
@@ -350,11 +357,22 @@ int unpack(const CopySpan *spans, int count, cudaStream_t s) {
 }  // namespace
 
 int copy_out(const CopySpan *spans, int count, cudaStream_t s) {
-  try {
-    return unpack(spans, count, s);
-  } catch (const std::bad_alloc &) {
-    return MDBAS_NB_ERR_ALLOC;
+  if (count > kMaxSpans) return MDBAS_NB_ERR_ARG;
+  Pool &p = pool();
+  std::unique_lock<std::mutex> lk(p.busy, std::try_to_lock);
+  if (lk.owns_lock() && p.plain < kPlainFirst) {
+    ++p.plain;
+    lk.unlock();
   }
+  int st;
+  try {
+    st = unpack(spans, count, s, lk.owns_lock() ? &p : nullptr);
+  } catch (const std::bad_alloc &) {
+    st = MDBAS_NB_ERR_ALLOC;
+  }
+  // copies on their way must not outlive the call, nor its hold on the slots
+  if (st != MDBAS_NB_OK) cudaStreamSynchronize(s);
+  return st;
 }
 
 void host_copy_enter() {

@@ -26,12 +26,16 @@ struct CopySpan3 {
           CopySpan(c, dev + 2 * n, sizeof(double) * n, add, true)} {}
 };
 
-// Host arrays to the device on stream s.  Returns when the host arrays have
-// been read; the device copies are ordered on s.
+// Host arrays to the device on stream s, ordered there.  Pageable arrays have
+// been read on return; page-locked ones are read by the copy engine and must
+// stay as they are until the stream has got there (every call of the drop-in
+// ends with a wait; of the engine's calls, those that return results do).
 // (Both take at most 16 spans.)
 int copy_in(const CopySpan *spans, int count, cudaStream_t s);
 // Device arrays to the host: waits for the work already on s and returns with
-// the data in the host arrays.
+// the data in the host arrays.  On an error their contents are undefined: work
+// that failed before the copies is noticed before anything is written, but a
+// device lost between two chunks leaves an array with `add` added to in part.
 int copy_out(const CopySpan *spans, int count, cudaStream_t s);
 
 // The page-locked chunks live while any user is registered (an engine, the

@@ -79,3 +79,49 @@ def test_round_trip_through_slots(gpu, n):
         for a, b in zip(e.positions(), (s.x, s.y, s.z)):
             assert np.array_equal(a, b)
     e.close()
+
+
+@pytest.mark.parametrize("n", [16383, 16384, 16386, 70002])
+def test_locked_and_pageable_in_one_result(gpu, n):
+    """Arrays on either side of the 128 KB from which page-locked ones are
+    written directly, past the results that are copied before the slots
+    exist."""
+    import torch
+    s = _atoms(n)
+    s.eps, s.sig = np.full(n, 1e-3), np.full(n, 1e-3)
+    e = _engine(s)
+    first = None
+    for k in range(14):
+        f = [torch.zeros(n, dtype=torch.float64).pin_memory().numpy() if (k >> a) & 1
+             else np.zeros(n) for a in range(3)]
+        en = e.evaluate(s.x, s.y, s.z, *f)
+        if first is None:
+            first = en, f
+        assert en == first[0]
+        for x, y in zip(f, first[1]):
+            assert np.array_equal(x, y)
+    e.close()
+
+
+# three arrays in one slot, ending inside a slot, over several slots, in all of
+# them, and in more than there are
+@pytest.mark.parametrize("n", [1001, 21846, 70001, 680001, 710001])
+def test_added_results(gpu, n):
+    """Forces added to the caller's: the old value plus the result, once."""
+    import ctypes as C
+    s = _atoms(n)
+    s.q = np.random.default_rng(2).uniform(-0.1, 0.1, n)
+    _, *ref, _ = nb.spme(s, grid=(32, 32, 32), nbsp=4)
+    assert np.abs(ref).max() > 0.0
+    pbc = nb.make_pbc(s.cell())
+    out = (C.c_double * 8)()
+    before = np.random.default_rng(3).uniform(-100, 100, (3, n))
+    hold = _engine(_atoms(1))  # the slots live
+    for _ in range(12):
+        f = [a.copy() for a in before]
+        nb.check(nb.lib().mdbas_nb_spme(n, C.byref(pbc), 0.34, systems.CHARGE_CONST, 32, 32, 32, 4,
+                                        *(nb._ptr(a) for a in (s.x, s.y, s.z, s.q, *f)), out, 0,
+                                        None), "spme")
+        for a, b, c in zip(f, before, ref):
+            assert np.array_equal(a, b + c)
+    hold.close()
