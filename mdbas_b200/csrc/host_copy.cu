@@ -53,21 +53,26 @@ constexpr int kMaxSpans = 16;
 constexpr size_t kLookFrom = (size_t)128 << 10;   // smaller arrays: staged even if page-locked
 
 // Helper threads that run one job at a time; a job is a function every
-// thread calls once, and returns from when nothing is left to take.
+// thread calls once, and returns from when nothing is left to take.  A job for
+// `helpers` threads is always for the same ones: taken in turn by all of three,
+// the lines of the caller's arrays move between their cores, and 2.3 MB took
+// 380 us where one thread's 110 are.
 class Helpers {
  public:
   void start(int helpers, void (*fn)(void *), void *arg) {
     {
       std::lock_guard<std::mutex> lk(m_);
       try {
-        while ((int)threads_.size() < helpers) threads_.emplace_back([this] { loop(); });
+        while ((int)threads_.size() < helpers)
+          threads_.emplace_back([this, k = (int)threads_.size()] { loop(k); });
       } catch (const std::exception &) {  // no more threads: with those there are
       }
       fn_ = fn;
       arg_ = arg;
-      room_ = helpers;
+      helpers_ = helpers;
+      ++job_;
     }
-    for (int k = 0; k < helpers; ++k) cv_.notify_one();
+    for (int k = 0; k < helpers; ++k) cv_[k].notify_one();
   }
   // No helper enters the job any more, and those inside have left it.
   void finish() {
@@ -80,19 +85,19 @@ class Helpers {
       std::lock_guard<std::mutex> lk(m_);
       stop_ = true;
     }
-    cv_.notify_all();
+    for (std::condition_variable &cv : cv_) cv.notify_one();
     for (std::thread &t : threads_) t.join();
     threads_.clear();
     stop_ = false;
   }
 
  private:
-  void loop() {
+  void loop(int k) {
     std::unique_lock<std::mutex> lk(m_);
-    for (;;) {
-      cv_.wait(lk, [&] { return stop_ || (fn_ && room_ > 0); });
+    for (unsigned long long done = job_ - 1;;) {
+      cv_[k].wait(lk, [&] { return stop_ || (fn_ && k < helpers_ && done != job_); });
       if (stop_) return;
-      --room_;
+      done = job_;
       auto *fn = fn_;
       void *arg = arg_;
       ++inside_;
@@ -103,11 +108,12 @@ class Helpers {
     }
   }
   std::mutex m_;
-  std::condition_variable cv_, idle_;
+  std::condition_variable cv_[kHelpers], idle_;  // cv_[k]: thread k's
   std::vector<std::thread> threads_;
   void (*fn_)(void *) = nullptr;
   void *arg_ = nullptr;
-  int room_ = 0;  // helpers that may still enter the job
+  int helpers_ = 0;             // threads that may enter the job
+  unsigned long long job_ = 1;  // its number; each thread enters once
   int inside_ = 0;
   bool stop_ = false;
 };
