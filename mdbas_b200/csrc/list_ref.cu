@@ -51,6 +51,7 @@ __constant__ short c_stencilOf[kInvSide * kInvSide * kInvSide];
 constexpr int kGroup = 8;       // atoms i per warp of the candidate tests
 constexpr int kListWarps = 4;   // warps per block of the list kernels
 constexpr int kPiece = 32;      // candidate chunks per warp of the tests
+constexpr int kTestWarps = 4096;  // of the tests before groups of atoms are split
 
 // image_update (src/utils.c:162-218), in place.
 __global__ void k_image_update(int n, DevBox b, double *x, double *y, double *z) {
@@ -182,17 +183,26 @@ __device__ __forceinline__ size_t table_row(int byStart, int cell, const int *ce
   return byStart ? cellStart[cell] : cell;
 }
 
-// Candidate chunks of every occupied cell, one warp per cell: chunkOff[l], the
-// first chunk of stencil cell l (its atoms in runs of 32), chunkOff[cellCheck]
-// the total, and chunkBase[c], the first position of chunk c.  A total beyond
-// stride raises FLAG_CELL and goes to *need.
+// Candidate chunks of every occupied cell, one warp per cell (byStart: per
+// atom, of which the first of its cell goes on): chunkOff[l], the first chunk of
+// stencil cell l (its atoms in runs of 32), chunkOff[cellCheck] the total, and
+// chunkBase[c], the first position of chunk c.  A total beyond stride raises
+// FLAG_CELL and goes to *need.
 __global__ void __launch_bounds__(32 * kListWarps)
 k_lc_chunks(int ncell, int nx, int ny, int nz, int cellCheck, int stride, int byStart,
-            const int *__restrict__ cellStart, int *__restrict__ chunkOff,
+            const int *__restrict__ cellStart, const int *__restrict__ cellOf,
+            const int *__restrict__ order, int *__restrict__ chunkOff,
             int *__restrict__ chunkBase, int *__restrict__ flags, int *__restrict__ need) {
   const int lane = threadIdx.x & 31;
-  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (k >= ncell || cellStart[k] == cellStart[k + 1]) return;
+  int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (byStart) {
+    const int p = k;
+    if (p >= cellStart[ncell]) return;
+    k = cellOf[order[p]];
+    if (cellStart[k] != p) return;
+  } else if (k >= ncell || cellStart[k] == cellStart[k + 1]) {
+    return;
+  }
   const int ix = k % nx, iy = (k / nx) % ny, iz = k / (nx * ny);
   const size_t row = table_row(byStart, k, cellStart);
   int *off = chunkOff + row * (cellCheck + 1);
@@ -230,11 +240,11 @@ k_lc_chunks(int ncell, int nx, int ny, int nz, int cellCheck, int stride, int by
 }
 
 // Where the candidates of atom p lie: chunks [first, last) of its mask row.
-// Link cells: atoms are tested in runs, the part of a group of kGroup
-// consecutive positions that lies in one cell; chunks of the own cell before
+// Link cells: atoms are tested in runs, the part of a group of `group` (at
+// most kGroup) consecutive positions that lies in one cell; chunks of the own cell before
 // the run hold no candidate.  All pairs: chunk c is atoms 32c .. 32c + 31.
 struct ChunkMap {
-  int linkCells, n, stride, cellCheck, ncell, byStart, nlc[3];
+  int linkCells, n, stride, cellCheck, ncell, byStart, group, nlc[3];
   const int *cellStart, *cellOf, *order, *posOf, *chunkOff, *chunkBase;
 
   __device__ __forceinline__ int atoms() const { return linkCells ? cellStart[ncell] : n; }
@@ -243,7 +253,7 @@ struct ChunkMap {
     return chunkOff + table_row(byStart, cell, cellStart) * (cellCheck + 1);
   }
   __device__ __forceinline__ void range(int p, int cell, int &first, int &last) const {
-    const int g0 = p & ~(kGroup - 1);
+    const int g0 = p & ~(group - 1);
     if (linkCells) {
       const int s = cellStart[cell];
       first = (max(g0, s) + 1 - s) >> 5;
@@ -284,7 +294,7 @@ __device__ __forceinline__ unsigned bits_after(int p, int base) {
   return s < 0 ? 0xffffffffu : s >= 31 ? 0u : 0xffffffffu << (s + 1);
 }
 
-// Candidate tests, link cells: one warp per group of kGroup positions in
+// Candidate tests, link cells: one warp per group of map.group positions in
 // [p0, p1) (p0 a multiple of kGroup) and piece of kPiece chunks (grid y); rows
 // of masks start at p0.
 // rl2 = (rc+delr)^2; band bounds the error of the FP32 r^2 near rl2.
@@ -299,8 +309,8 @@ k_lc_masks(int p0, int p1, DevBox b, ChunkMap map, double cutnb2, float rl2, flo
            const double *__restrict__ zs, const float4 *__restrict__ cs,
            const int *__restrict__ flags, unsigned *__restrict__ masks) {
   const int lane = threadIdx.x & 31;
-  const int g0 = p0 + kGroup * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int end = min(min(g0 + kGroup, p1), map.atoms());
+  const int g0 = p0 + map.group * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int end = min(min(g0 + map.group, p1), map.atoms());
   if (g0 >= end || (*flags & FLAG_CELL)) return;
   const int nx = map.nlc[0], ny = map.nlc[1], nz = map.nlc[2];
   for (int p = g0; p < end;) {
@@ -395,13 +405,28 @@ k_lc_masks(int p0, int p1, DevBox b, ChunkMap map, double cutnb2, float rl2, flo
         if ((c & 3) == 3) words.flush(lane, c, atoms, rows, map.stride);
       }
     };
-    int l = 0;
-    while (l < map.cellCheck && off[l + 1] <= c) ++l;
-    if (l == 0 && c < cLast) {
+    // the stencil cell that chunk c lies in, 32 at a time from cell l on (one
+    // after the other they are latency: 20,000 atoms spread over 300 A at link
+    // ratio 3, of whose 156 stencil cells 11 hold atoms, 673 -> 442 us; 96,000
+    // atoms of water at ratio 5 11.1 -> 7.4 ms, at ratio 1 no change)
+    const auto holding = [&](int l) {
+      for (; l < map.cellCheck; l += 32) {
+        const int k = l + lane;
+        const unsigned m =
+            __ballot_sync(0xffffffffu, k < map.cellCheck && off[k + 1] > c);
+        if (m) return l + __ffs(m) - 1;
+      }
+      return l;
+    };
+    int l = holding(0);
+    if (l == 0) {
       scan(0, std::true_type{});
       l = 1;
     }
-    for (; l < map.cellCheck && c < cLast; ++l) scan(l, std::false_type{});
+    for (; l < map.cellCheck && c < cLast; ++l) {
+      if (off[l + 1] <= c) l = holding(l + 1);
+      if (l < map.cellCheck) scan(l, std::false_type{});
+    }
     if (c & 3) words.flush(lane, c, atoms, rows, map.stride);
     p += atoms;
   }
@@ -694,6 +719,7 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
   ChunkMap map{};
   map.linkCells = linkCells;
   map.n = n;
+  map.group = kGroup;
   int ratio = 1;
   if (linkCells) {
     MDB_TRY(load_stencil());
@@ -709,6 +735,13 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
     // chunks per cell of evenly spread atoms with room for fluctuations; a
     // denser cell reports what it needs and the build is made again
     const double per = (double)n / w.ncell;
+    // Groups that mostly span cells are a warp's runs one after the other:
+    // with few atoms and pieces they are split, until there are kTestWarps
+    // warps (2,000 atoms spread over 100 A, link ratio 2: 204 -> 111 us, over
+    // 200 A 144 -> 108; 3,000 atoms of water at ratio 5, where the pieces make
+    // enough, would take 432 instead of 369)
+    const double warps = n * std::max(1., map.cellCheck * std::min(1., per) / kPiece);
+    while (map.group > 1 && warps < kTestWarps * map.group && per < map.group) map.group /= 2;
     map.stride = map.cellCheck * (int)((1.25 * per + 3. * sqrt(per)) / 32. + 1.);
     map.stride = (std::max(map.stride, w.maskStride) + 3) & ~3;
   } else {
@@ -766,10 +799,10 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
                  w.order.as<int>(), w.xu.as<double>(), w.yu.as<double>(), w.zu.as<double>(),
                  frozen, w.xs.as<double>(), w.ys.as<double>(), w.zs.as<double>(),
                  w.cs.as<float4>(), w.posOf.as<int>());
-      MDB_LAUNCH(k_lc_chunks, grid_for(ncell, kListWarps), 32 * kListWarps, 0, s, ncell, w.nlc[0],
-                 w.nlc[1], w.nlc[2], map.cellCheck, map.stride, map.byStart,
-                 w.cellStart.as<int>(), w.chunkOff.as<int>(), w.chunkBase.as<int>(), flags,
-                 flags + 1);
+      MDB_LAUNCH(k_lc_chunks, grid_for((long long)tableRows, kListWarps), 32 * kListWarps, 0, s,
+                 ncell, w.nlc[0], w.nlc[1], w.nlc[2], map.cellCheck, map.stride, map.byStart,
+                 w.cellStart.as<int>(), w.cellOf.as<int>(), w.order.as<int>(),
+                 w.chunkOff.as<int>(), w.chunkBase.as<int>(), flags, flags + 1);
     } else {
       const double bx = b.a1, by = b.type == CUBIC ? b.a1 : b.b2,
                    bz = b.type == CUBIC ? b.a1 : b.c3;
@@ -795,7 +828,7 @@ int build_ref_list(RefListWork &w, int n, const DevBox &b, double cutOff, double
     MDB_TRY(w.masks.ensure(sizeof(unsigned) * (size_t)map.stride * std::min<long long>(slab, n)));
     const auto test = [&](int p0, int p1) -> int {
       unsigned *m = w.masks.as<unsigned>();
-      const int g = grid_for(p1 - p0, kGroup * kListWarps);
+      const int g = grid_for(p1 - p0, map.group * kListWarps);
       if (linkCells) {
         const auto kern = frozen ? k_lc_masks<true> : k_lc_masks<false>;
         MDB_LAUNCH(kern, dim3(g, grid_for(map.stride, kPiece)), 32 * kListWarps, 0, s, p0, p1, b,
