@@ -375,7 +375,8 @@ int mdbas_nb_engine_set_topology(mdbas_nb_engine *e, const double *q, const doub
                                  const double *sig, const int *frozen, const int *exclPair,
                                  const int *exclFlat);
 /* Positions: host pointers (copied H2D on the engine stream) or device
- * pointers (device != 0), FP64, original atom order. */
+ * pointers (device != 0), FP64, original atom order.  Page-locked host arrays
+ * must stay unchanged until a call that returns results has been made. */
 int mdbas_nb_engine_set_positions(mdbas_nb_engine *e, const double *x, const double *y,
                                   const double *z, int device_ptrs);
 /* Sort atoms into cells/clusters and build the cluster-pair list (precision 1)

@@ -18,7 +18,7 @@
 //
 // Measured (B200, 16-core virtual host), the caller's arrays touched before:
 // 72 KB of forces 70 -> 39 us, 2.3 MB 240 -> 139 us; makelist and energy of
-// 18,558 atoms (a 43 MB list) 5.5 -> 3.1 ms.  Helpers: one up to 8 MB (2.3 MB:
+// 18,558 atoms (a 43 MB list) 5.5 -> 3.1 to 3.7 ms.  Helpers: one up to 8 MB (2.3 MB:
 // 139 us, with two 154, with none 211), three beyond (five: no better); none
 // for results that are added to the caller's arrays, whose pages are often
 // new (every thread's page faults interrupt the others: an SPME call of

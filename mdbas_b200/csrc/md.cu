@@ -1144,6 +1144,11 @@ int md_prune_sync(mdbas_nb_engine *e) {
 // words, the bonded terms and the exclusions.  (A branch each: no faster, and
 // the graph of 20 steps took 6.6 ms to instantiate with SPME
 // and bonded terms, 3.7 without, against 5.2 and 2.6.)
+// The branches make the graph dearer to instantiate and to destroy: a new
+// engine's first 40 steps and its end took 7.6 + 3.2 ms before them and take
+// 7.6 + 4.0 at 3,000 atoms of water, 7.9 + 4.8 and 8.7 + 7.8 with 10,000 atoms of
+// chains without SPME, which their shorter steps pay back in 40 and 120 steps
+// more.  (Without BR_SIDE 6.4 + 2.7 and 6.4 + 4.4, but 4 % and 16 % a step.)
 enum MdBranch { BR_KSPACE = 0, BR_SIDE = 1 };
 
 int md_fork(mdbas_nb_engine *e, MdBranch b, cudaStream_t s) {

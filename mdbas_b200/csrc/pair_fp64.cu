@@ -11,9 +11,8 @@
 // This translation unit is compiled with --fmad=false.  Distances, the cut-off
 // test and the general pair form keep MDBas's association order; the Ewald
 // pairs of the ordinary range take the Newton and polynomial forms of
-// real64.cuh (a few ulp from the C library's; the forces of a 3,000-atom
-// water box are 1.98e-15 from a long-double sum, 2.15e-15 with the C
-// library's).  The order of the FP64 additions is not fixed.
+// real64.cuh (a few ulp from the C library's; no further from exact).  The
+// order of the FP64 additions is not fixed.
 #include "common.cuh"
 #include "pair_fp64.cuh"
 #include "pair_rows.cuh"
@@ -199,8 +198,8 @@ __device__ __forceinline__ void exact_finish(double *acc, int c) {
 // over all their atoms.  Bound by latency and the LSU (gathers and scattered
 // additions, 60% of the data-pipe cycles; FP64 pipe 40%).  Measured against
 // one thread per atom with the C library's functions: 2.26 -> 0.67 ms at
-// 96,000 atoms of water, 1.22 -> 0.10 at 12,000, 1.23 -> 0.046 at 3,000.
-// Atoms packed to one 32-byte sector and j forces added a sector at a time
+// 96,000 atoms of water, 1.22 -> 0.10 at 12,000, 1.23 -> 0.046 at 3,000 (calls
+// in a row, L2 warm; 0.79 at 96,000 after an L2 flush).  Atoms packed to one 32-byte sector and j forces added a sector at a time
 // measured no better (0.67 and 1.1 ms).
 template <bool EWALD>
 __global__ void __launch_bounds__(32 * kRowWarps, kPairBlocks)

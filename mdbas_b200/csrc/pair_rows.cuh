@@ -7,7 +7,7 @@
 // time, so the FP64 arithmetic runs with full warps (62% of a 14 A list lies
 // within 12 A).  The walk is bound by latency: entries are loaded two rounds
 // ahead and positions one round ahead (the 96,000-atom pair loop 0.93 -> 0.67
-// ms), and atoms are handed out by a counter, the next one fetched while the
+// ms, L2 warm), and atoms are handed out by a counter, the next one fetched while the
 // current one runs.  A row can be cut into 2^split work items, so that a
 // small system fills the SMs.
 #pragma once

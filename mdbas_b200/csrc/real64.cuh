@@ -3,9 +3,12 @@
 //
 // The pair kernels are bound by the FP64 pipe.  sqrt, three divisions, erfc and
 // exp of the C library forms cost about 250 FP64 instructions per pair; the
-// forms here about 60, with the same accuracy in the sums (the measured error
-// of the forces against 64-bit torch is unchanged).  They hold on the range
-// that pair_fast accepts; pairs outside it take the library forms.
+// forms here about 60.  A pair's energy and force are within 6 x 2^-53 of exact
+// (1.4 rms; tests/test_gpu_pair_functions.py); the forces of eight 3,000-atom
+// boxes of water are 2.76e-15 from long double sums (with the library's
+// functions 2.86e-15), their energies 2.3e-10 internal units (3.5e-10).  They
+// hold on the range that the callers check; pairs outside it take the library
+// forms.
 #pragma once
 
 #include "common.cuh"

@@ -14,7 +14,8 @@ relative error (2.4e-8).
 
 fit64 derives the FP64 form of csrc/real64.cuh: (x + 3) erfcx(x) as a
 polynomial of degree 18 in t = (x - 3) / (x + 3), x in [0, 6], by Chebyshev
-interpolation.  erfcx comes from the power series of erf (x < 5) or the
+interpolation; the map is that of Shepherd and Laframboise (Math. Comp. 36
+(1981) 249), who take (1 + 2 x) erfcx(x) over [0, inf).  erfcx comes from the power series of erf (x < 5) or the
 continued fraction of erfc, in 70-digit decimal arithmetic; the interpolation
 error is 1.9e-17 relative.
 """
